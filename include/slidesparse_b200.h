@@ -285,6 +285,10 @@ int ss_plan_run(int64_t handle, const void* x_bf16, int64_t x_row_stride,
  * csrc/graph_projection.cuh:159-163 (release). */
 int ss_plan_release(int64_t handle);
 
+/* out[0..5] = {device, m, k, n, padded m, padded lifted k} of a plan, for bindings that check an
+ * input against it.  csrc/graph_projection.cuh:92-98 (the checks of Plan::forward). */
+int ss_plan_shape(int64_t handle, int64_t* out, int n_out);
+
 /* out[0..7] = {threads, dynamic smem bytes, registers, local bytes, CTAs/SM, token tile,
  * smem stages, TMEM columns}.  csrc/graph_projection.cuh:85-89,176 (resources). */
 int ss_plan_resources(int64_t handle, int64_t* out, int n_out);

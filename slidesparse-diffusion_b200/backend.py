@@ -3,7 +3,10 @@
 Host-side mirror of `sdacc/w8a8_slidesparse/backend.py` (build_native :17-70, load_native
 :73-118).  The native artefact is a thin C-ABI shared library (include/slidesparse_b200.h) built
 with nvcc for sm_100a only -- no CUTLASS, no Triton, no second backend, no CPU fallback: every
-operator below raises if the library is missing.
+operator below raises if the library is missing.  Beside it lies a second library built by the host
+compiler from csrc/ss_torch.cpp, which binds the operators of the forward path to that C ABI without
+going through Python (an eager call took 33-40 us of host time through ctypes); a directory that
+holds the C library alone binds the same operators through ctypes.
 
 The operators keep the reference's names and schemas (csrc/dualscale_sm80.cu:400-406,
 csrc/projection_sm80.cu:154-169, csrc/graph_projection.cuh:178-195) so callers that look them up
@@ -23,6 +26,8 @@ from .packing import group_size, lifted_k
 
 SS_E_ARG, SS_E_CUDA, SS_E_FORMAT, SS_E_HANDLE, SS_E_DEVICE, SS_E_LIMIT = -1, -2, -3, -4, -5, -6
 LIBRARY_NAME = "libslidesparse_b200.so"
+BINDING_LIBRARY_NAME = "libslidesparse_b200_torch.so"
+BINDING_SOURCE = "ss_torch.cpp"
 SOURCES = ("ss_api.cu", "ss_gemm.cu", "ss_frontend.cu", "ss_pack.cu", "ss_noalloc.cu", "ss_micro.cu", "ss_obs.cu")
 ARCH = "sm_100a"
 VALID_CONFIGS = (0, 1, 2, 3, 4, 5, 6, 11, 12, 13, 14, 15, 16, 17)
@@ -44,7 +49,7 @@ def default_directory():
 
 def _source_identity():
     csrc = _PACKAGE / "csrc"
-    files = sorted(p for p in csrc.iterdir() if p.suffix in (".cu", ".cuh"))
+    files = sorted(p for p in csrc.iterdir() if p.suffix in (".cu", ".cuh", ".cpp"))
     files.append(_PACKAGE.parent / "include" / "slidesparse_b200.h")
     return {p.name: sha(p) for p in files}
 
@@ -53,9 +58,9 @@ def build_native(output=None, arch=ARCH, force=False):
     """Offline build, without initialising CUDA; call before measurement.
 
     Compiles csrc/*.cu into <output>/libslidesparse_b200.so with
-    `nvcc -gencode arch=compute_100a,code=sm_100a` and writes receipt.json (source / library
-    hashes, torch and CUDA versions, the command).  Returns the receipt.  An up-to-date artefact
-    is kept unless force=True.
+    `nvcc -gencode arch=compute_100a,code=sm_100a`, csrc/ss_torch.cpp into the operator binding beside
+    it with the host compiler, and writes receipt.json (source / library hashes, torch and CUDA
+    versions, the command).  Returns the receipt.  An up-to-date artefact is kept unless force=True.
     """
     if torch.cuda.is_initialized():
         raise RuntimeError("build in a fresh CPU-only process")
@@ -63,25 +68,36 @@ def build_native(output=None, arch=ARCH, force=False):
         raise ValueError("this library is written for sm_100a only")
     output = Path(output) if output is not None else default_directory()
     output.mkdir(parents=True, exist_ok=True)
-    target, receipt_path = output / LIBRARY_NAME, output / "receipt.json"
+    target, binding, receipt_path = output / LIBRARY_NAME, output / BINDING_LIBRARY_NAME, output / "receipt.json"
     identity = _source_identity()
-    if not force and target.exists() and receipt_path.exists():
+    if not force and target.exists() and binding.exists() and receipt_path.exists():
         old = json.loads(receipt_path.read_text())
-        if old.get("complete") and old.get("source_dependencies") == identity and old.get("library_sha") == sha(target):
+        if (old.get("complete") and old.get("source_dependencies") == identity and old.get("library_sha") == sha(target)
+                and old.get("binding_sha") == sha(binding)):
             return old
     nvcc = str(Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "bin/nvcc")
     cmd = [nvcc, "-std=c++17", "-O3", "--shared", "-Xcompiler", "-fPIC", "-lineinfo", "-Xptxas=-v",
-           "-gencode", "arch=compute_100a,code=sm_100a"]
+           "--threads", "0", "-gencode", "arch=compute_100a,code=sm_100a"]
     cmd += [str(_PACKAGE / "csrc" / name) for name in SOURCES]
     cmd += ["-o", str(target)]
     log = output / "compile.log"
     with log.open("w") as f:
         subprocess.run(cmd, check=True, stdout=f, stderr=subprocess.STDOUT)
-    receipt = dict(complete=True, arch=arch, library_sha=sha(target), source_dependencies=identity,
+        subprocess.run(_binding_command(output, binding), check=True, stdout=f, stderr=subprocess.STDOUT)
+    receipt = dict(complete=True, arch=arch, library_sha=sha(target), binding_sha=sha(binding), source_dependencies=identity,
                    torch=torch.__version__, cuda=torch.version.cuda, command=cmd,
                    compile_log_sha=sha(log), cuda_initialized=torch.cuda.is_initialized())
     receipt_path.write_text(json.dumps(receipt, indent=2) + "\n")
     return receipt
+
+
+def _binding_command(directory, target):
+    """The host compiler's command for the operator binding, linked to the C library next to it."""
+    root, cuda = Path(torch.__file__).parent, Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    include = [root / "include", root / "include/torch/csrc/api/include", cuda / "include"]
+    return ([os.environ.get("CXX", "g++"), "-std=c++17", "-O2", "-shared", "-fPIC"] + [f"-I{path}" for path in include]
+            + [str(_PACKAGE / "csrc" / BINDING_SOURCE), f"-L{directory}", "-lslidesparse_b200", f"-L{root / 'lib'}",
+               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-Wl,-rpath,$ORIGIN", "-o", str(target)])
 
 
 BINDING_NAME = "SOURCE_BINDING.json"
@@ -96,7 +112,7 @@ def source_binding_files(directory=None):
         rel = path.relative_to(root)
         if not path.is_file() or rel.parts[0].startswith("native_") or "__pycache__" in rel.parts:
             continue
-        if path.name != BINDING_NAME and path.suffix in (".py", ".json", ".cu", ".cuh"):
+        if path.name != BINDING_NAME and path.suffix in (".py", ".json", ".cu", ".cuh", ".cpp"):
             names.append(rel.as_posix())
     return names
 
@@ -140,6 +156,7 @@ def _declare(lib):
         "ss_plan_create": [vp, vp, vp, vp, i64, i64, i64, i64, i32, vp],
         "ss_plan_run": [i64, vp, i64, vp, vp, vp, i64, vp],
         "ss_plan_release": [i64],
+        "ss_plan_shape": [i64, vp, i32],
         "ss_plan_resources": [i64, vp, i32],
         "ss_gemm_resources": [i64, i64, i64, vp, i32],
         "ss_device_status": [vp, vp],
@@ -178,9 +195,12 @@ def load_native(directory=None):
         if _loaded_sha != receipt["library_sha"]:
             raise RuntimeError("a different native binary is already loaded in this process")
         return receipt
+    binding = directory / BINDING_LIBRARY_NAME
+    if binding.exists() and receipt.get("binding_sha") != sha(binding):
+        raise ValueError("operator binding differs from its receipt")
     _lib = _declare(ctypes.CDLL(str(target)))
     _loaded_sha = receipt["library_sha"]
-    _register_ops()
+    _register_ops(binding if binding.exists() else None)
     return receipt
 
 
@@ -691,7 +711,9 @@ def check_device(device=None):
 _libraries = []
 
 
-def _register_ops():
+def _register_ops(binding):
+    """Define the operators and their fake kernels; `binding` (path of the native operator binding)
+    implements the forward path, without one the ctypes functions above do."""
     global _ops_registered
     if _ops_registered:
         return
@@ -705,7 +727,6 @@ def _register_ops():
                 "int config,Tensor? output_addend=None)->Tensor")
     dual.impl("pack_cpu", lambda weight, padded_k: pack_weight(weight, padded_k), "CPU")
     dual.impl("configure", _configure, "CUDA")
-    dual.impl("run", _run, "CUDA")
 
     mild = Library("sdacc_mild_projection_sm80", "DEF")
     proj = ("(Tensor input,Tensor packed,Tensor metadata,Tensor scales,Tensor bias,int group,int n,int config,"
@@ -716,12 +737,6 @@ def _register_ops():
     mild.define("quantize_scalar(Tensor input)->(Tensor,Tensor)")
     mild.define("projection" + proj)
     mild.define("projection_scalar" + proj)
-    # One front-end serves all three reference variants: they produce identical bits.
-    mild.impl("quantize", _quantize, "CUDA")
-    mild.impl("quantize_packed16", _quantize, "CUDA")
-    mild.impl("quantize_scalar", lambda input: _quantize(input, 4), "CUDA")
-    for name in ("projection", "projection_packed16", "projection_scalar"):
-        mild.impl(name, _projection, "CUDA")
 
     prepared = Library("sdacc_prepared_projection_sm80", "DEF")
     prep = ("(Tensor packed,Tensor metadata,Tensor scales,Tensor bias,int k,int m,int n,int group,int config,"
@@ -732,7 +747,6 @@ def _register_ops():
     prepared.define("resources(int handle)->int[]")
     prepared.define("run(Tensor input,int handle,int n)->Tensor")
     prepared.define("release(int handle)->()")
-    prepared.impl("run", _prepared_run, "CUDA")
     prepared.impl("release", _release, "CompositeExplicitAutograd")
     prepared.impl("resources", _resources, "CompositeExplicitAutograd")
     _libraries.extend([dual, mild, prepared])
@@ -771,8 +785,19 @@ def _register_ops():
         _projection_fused_impl(input, _prologue_of(prologue, shift, scale, eps), packed, metadata, scales, bias, group, n,
                                None, gate, residual)
 
-    own.impl("projection_fused", _op_fused, "CUDA")
-    own.impl("projection_fused_accumulate_", _op_fused_accumulate, "CUDA")
+    if binding is not None:
+        torch.ops.load_library(str(binding))
+    else:
+        dual.impl("run", _run, "CUDA")
+        # One front-end serves all three reference variants: they produce identical bits.
+        mild.impl("quantize", _quantize, "CUDA")
+        mild.impl("quantize_packed16", _quantize, "CUDA")
+        mild.impl("quantize_scalar", lambda input: _quantize(input, 4), "CUDA")
+        for name in ("projection", "projection_packed16", "projection_scalar"):
+            mild.impl(name, _projection, "CUDA")
+        prepared.impl("run", _prepared_run, "CUDA")
+        own.impl("projection_fused", _op_fused, "CUDA")
+        own.impl("projection_fused_accumulate_", _op_fused_accumulate, "CUDA")
     _libraries.append(own)
 
     @torch.library.register_fake("slidesparse_b200::projection_fused")

@@ -265,6 +265,15 @@ extern "C" int ss_plan_release(int64_t handle) {
   return SS_OK;
 }
 
+extern "C" int ss_plan_shape(int64_t handle, int64_t* out, int n_out) {
+  auto plan = find_plan(handle);
+  SS_REQUIRE(plan, SS_E_HANDLE, "prepared handle %lld absent", (long long)handle);
+  SS_REQUIRE(out && n_out >= 6, SS_E_ARG, "plan_shape: out must hold 6 values");
+  out[0] = plan->device; out[1] = plan->m; out[2] = plan->k;
+  out[3] = plan->n; out[4] = plan->pm; out[5] = plan->pk;
+  return SS_OK;
+}
+
 extern "C" int ss_plan_resources(int64_t handle, int64_t* out, int n_out) {
   auto plan = find_plan(handle);
   SS_REQUIRE(plan, SS_E_HANDLE, "prepared handle %lld absent", (long long)handle);
