@@ -123,8 +123,12 @@ quant_lift_kernel(const uint16_t* __restrict__ x, int64_t sx, int8_t* __restrict
   __shared__ float warp_fmax[32];
   __shared__ float s_inv;
   __shared__ uint32_t s_bits;
-  // lets a GEMM launched with programmatic stream serialization run its set-up while the last
-  // wave of rows is still being quantised (it waits on the device before reading q or sa)
+  // Launched with programmatic stream serialization: the CTAs may be placed while the kernel before
+  // this one still runs, and wait here for it to complete before x is read or q written.  Only then
+  // is the GEMM that follows let in (its set-up and weight fetch run while the last wave of rows is
+  // still being quantised; it waits on the device before reading q or sa): weights written by an
+  // earlier kernel of the stream are complete by then.
+  ptx::grid_dep_wait();
   ptx::grid_dep_launch();
 
   const int row = blockIdx.x, t = threadIdx.x, T = blockDim.x;
@@ -315,8 +319,17 @@ int launch_one(const void* x, int64_t sx, int m, int k, int pm, int pk, int8_t* 
   const int threads = ((chunks + kChunks - 1) / kChunks + 31) / 32 * 32;
   SS_REQUIRE(threads <= kMaxThreads, SS_E_LIMIT, "front-end: K=%d beyond the supported %d", k,
              kMaxThreads * kMaxVec * 8);
-  quant_lift_kernel<L, VEC, PRO><<<pm, threads, 0, stream>>>(static_cast<const uint16_t*>(x), sx, q, sa, m, k, pk, nvec, chunks, pro);
-  SS_CUDA(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(pm);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = options().pdl ? 1 : 0;
+  SS_CUDA(cudaLaunchKernelEx(&cfg, quant_lift_kernel<L, VEC, PRO>, static_cast<const uint16_t*>(x), sx, q, sa, m, k, pk, nvec,
+                             chunks, pro));
   return SS_OK;
 }
 
