@@ -191,6 +191,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
+// The same wait for a whole warp: the lanes leave together, by a vote, so that the compiler keeps what
+// follows on warp-uniform registers.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
+                                               unsigned long long limit_ns = kDefaultWaitNs) {
+  if (__any_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  uint64_t deadline = 0;
+  for (uint32_t spin = 1;; ++spin) {
+    if (__any_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    if ((spin & 0x3fu) == 0) {
+      const uint64_t now = globaltimer_ns();
+      if (deadline == 0) deadline = now + limit_ns;
+      else if (__all_sync(0xffffffffu, now > deadline)) return false;
+    }
+  }
+}
+
 // TMA tiled loads (no multicast anywhere in this library).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar,
                                             int x, int y) {

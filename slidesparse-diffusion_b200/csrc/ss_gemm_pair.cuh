@@ -235,7 +235,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   static_assert(!RES || T::kAccBufs == 2, "resident form assumes two accumulators");
   static_assert(!(T::kHalfTail && MODE == kOutBf16TmaPeers), "the tensor-parallel stores take whole chunks only");
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int tiles_ch2 = (args.tiles_ch + 1) >> 1;            // tiles of 256 channels
@@ -292,7 +292,8 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     // three lanes issuing one each in the same warp instruction cost the same as one lane issuing
     // three, so the count per stage is what matters: with five (one per 128-column block and
     // operand) this thread set the pace of the whole pipeline.
-    if (lane == 0) {
+    {
+      const bool leader = ptx::elect_one();
       uint32_t s = 0, phase = 0;       // pipeline stage and the parity of its current use
       uint32_t issued = 0, tl = 0;     // stages filled so far
       bool ok = true;
@@ -303,13 +304,14 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         // the weights do not depend on the preceding kernel: fetch the resident operands first
         if (tile_first < num_tiles) {
           const int ch0 = (tile_first % tiles_ch2) * (2 * kTileCh) + static_cast<int>(rank) * kTileCh;
-          if (rank == 0) ptx::mbar_arrive_expect_tx(&bar_meta[1], 2 * num_st * (T::kABytes + T::kEBytes));
-          for (int st = 0; st < num_st; ++st) {
+          if (leader && rank == 0) ptx::mbar_arrive_expect_tx(&bar_meta[1], 2 * num_st * (T::kABytes + T::kEBytes));
+          for (int st = 0; st < num_st && leader; ++st) {
             ptx::tma_load_2d_pair(smem + off_a + st * T::kABytes, &map_a, &bar_meta[1], st * KB * (kBlockK / 2), ch0);
             // the metadata is staged where the first activation stages will live
             ptx::tma_load_3d_pair(smem + off_e + st * T::kEBytes, &map_e, &bar_meta[1], 0, ch0 >> 5, st * KB);
           }
-          if (!ptx::mbar_wait(&bar_meta[0], 0, args.wait_ns)) ok = false;
+          __syncwarp();
+          if (!ptx::mbar_wait_warp(&bar_meta[0], 0, args.wait_ns)) ok = false;
         }
       }
       ptx::grid_dep_wait();           // q is written by the kernel launched just before this one
@@ -319,24 +321,27 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         SS_TL(0, tl, 0);
         for (int st = w.s0; st < w.s1; ++st) {
           SS_PF_BEGIN();
-          if (!ptx::mbar_wait(&bar_empty[s], phase ^ 1u, args.wait_ns)) { ok = false; break; }
+          if (!ptx::mbar_wait_warp(&bar_empty[s], phase ^ 1u, args.wait_ns)) { ok = false; break; }
           SS_PF(pf_wait);
-          if (rank == 0) {
-            if constexpr (!RES) ptx::mbar_arrive_expect_tx(&bar_e[s], 2u * T::kEBytes);
-            ptx::mbar_arrive_expect_tx(&bar_full[s], kStageTx);
+          if (leader) {
+            if (rank == 0) {
+              if constexpr (!RES) ptx::mbar_arrive_expect_tx(&bar_e[s], 2u * T::kEBytes);
+              ptx::mbar_arrive_expect_tx(&bar_full[s], kStageTx);
+            }
+            SS_PF(pf_arm);
+            if constexpr (!RES) {
+              // the metadata first: it is small, and its copy into TMEM can start while the rest lands
+              ptx::tma_load_3d_pair(smem + off_e + s * T::kEBytes, &map_e, &bar_e[s], 0, ch0 >> 5, st * KB);
+              SS_PF(pf_e);
+            }
+            ptx::tma_load_3d_pair(smem + off_b + s * T::kBBytes, &map_b, &bar_full[s], 0, tok0, st * KB);
+            SS_PF(pf_b);
+            if constexpr (!RES) {
+              ptx::tma_load_2d_pair(smem + off_a + s * T::kABytes, &map_a, &bar_full[s], st * KB * (kBlockK / 2), ch0);
+              SS_PF(pf_a);
+            }
           }
-          SS_PF(pf_arm);
-          if constexpr (!RES) {
-            // the metadata first: it is small, and its copy into TMEM can start while the rest lands
-            ptx::tma_load_3d_pair(smem + off_e + s * T::kEBytes, &map_e, &bar_e[s], 0, ch0 >> 5, st * KB);
-            SS_PF(pf_e);
-          }
-          ptx::tma_load_3d_pair(smem + off_b + s * T::kBBytes, &map_b, &bar_full[s], 0, tok0, st * KB);
-          SS_PF(pf_b);
-          if constexpr (!RES) {
-            ptx::tma_load_2d_pair(smem + off_a + s * T::kABytes, &map_a, &bar_full[s], st * KB * (kBlockK / 2), ch0);
-            SS_PF(pf_a);
-          }
+          __syncwarp();
           if (++s == static_cast<uint32_t>(kRing)) { s = 0; phase ^= 1u; }
           ++issued;
         }
@@ -344,7 +349,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       }
       SS_PF_STORE(0, pf_wait); SS_PF_STORE(1, pf_arm); SS_PF_STORE(2, pf_a); SS_PF_STORE(3, pf_b); SS_PF_STORE(4, pf_e);
       SS_PF_STORE(5, static_cast<long long>(issued));
-      if (!ok) {
+      if (!ok && leader) {
         atomicOr(args.status, kStatusProducerTimeout);
         // Let the copies already in flight land before the pair's shared memory is released.  The
         // full barriers live in rank 0 and count both CTAs' bytes, so rank 0 waits (bounded) for the
@@ -368,7 +373,8 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     // polls, commits) is time the pipe stands idle.  The ring is therefore unrolled with the stage
     // slot as a compile-time constant: every shared-memory descriptor is one add away from a
     // value computed before the loop, and a stage costs four MMAs, one commit and one barrier poll.
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
+      const bool leader = ptx::elect_one();
       constexpr uint32_t idesc = (1u << 2) | (2u << 4) | (1u << 7) | (1u << 10) |
                                  (static_cast<uint32_t>(NT >> 3) << 17) |
                                  (static_cast<uint32_t>((2 * kTileCh) >> 4) << 24);
@@ -395,18 +401,18 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       if constexpr (RES) {
         // once per cluster: metadata of the whole K extent from its staging area into TMEM
         if (more) {
-          if (!ptx::mbar_wait(&bar_meta[1], 0, args.wait_ns)) ok = false;
+          if (!ptx::mbar_wait_warp(&bar_meta[1], 0, args.wait_ns)) ok = false;
           ptx::tc_fence_after();
           const uint32_t e_addr = ptx::smem_u32(smem + off_e);
           const uint32_t e_tmem = tmem_base + T::kMetaCol;
-          for (int kb = 0; kb < args.num_kb && ok; kb += 2) {
+          for (int kb = 0; kb < args.num_kb && ok && leader; kb += 2) {
             if (kb + 1 < args.num_kb && args.wide_cp)
               ptx::tc_cp_128x256b_pair(e_tmem + 4 * kb, smem_desc(e_addr + kb * T::kEBlock, T::kEBlock, 128, 0));
             else
               for (int h = kb; h < kb + 2 && h < args.num_kb; ++h)
                 ptx::tc_cp_128x128b_pair(e_tmem + 4 * h, smem_desc(e_addr + h * T::kEBlock, 128, 128, 0));
           }
-          ptx::tc_commit_pair(&bar_meta[0], 3);       // both producers: the staging area is free
+          if (leader) ptx::tc_commit_pair(&bar_meta[0], 3);       // both producers: the staging area is free
         }
       }
       if (probe) probe_begin = clock64();
@@ -414,7 +420,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       uint32_t buf = 0, d_tmem = tmem_base;
       if (more && ok) {
         SS_TL(1, tl, 0);
-        if (!ptx::mbar_wait(&bar_acc_empty[0], 1u, args.wait_ns)) ok = false;
+        if (!ptx::mbar_wait_warp(&bar_acc_empty[0], 1u, args.wait_ns)) ok = false;
         SS_TL(1, tl, 1);
         ptx::tc_fence_after();
       }
@@ -422,10 +428,10 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
 #pragma unroll
         for (int slot = 0; slot < kRing; ++slot) {
           SS_PF_BEGIN();
-          if (!ptx::mbar_wait(&bar_full[slot], phase, args.wait_ns)) { ok = false; more = false; break; }
+          if (!ptx::mbar_wait_warp(&bar_full[slot], phase, args.wait_ns)) { ok = false; more = false; break; }
           if constexpr (!RES) {
             // without a metadata warp this thread copies the stage's metadata itself (below)
-            if (!meta_warp && !ptx::mbar_wait(&bar_e[slot], phase, args.wait_ns)) { ok = false; more = false; break; }
+            if (!meta_warp && !ptx::mbar_wait_warp(&bar_e[slot], phase, args.wait_ns)) { ok = false; more = false; break; }
           }
           SS_PF(pf_ready);
           if (st == st_first) SS_TL(1, tl, 2);
@@ -436,7 +442,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           const uint32_t b_lo = b_lo0 + static_cast<uint32_t>(slot) * (T::kBBytes >> 4);
           const uint32_t e_tmem = tmem_base + T::kMetaCol + static_cast<uint32_t>(RES ? st : slot) * T::kMetaColsPerStage;
           const bool full_stage = !(odd_tail && st == num_st - 1);
-          if (!RES && !meta_warp) {
+          if (!RES && !meta_warp && leader) {
             // no metadata warp (three pipeline stages): this thread copies the stage's metadata itself
             const uint32_t e_addr = ptx::smem_u32(smem + off_e) + slot * T::kEBytes;
             if (KB == 2 && full_stage && args.wide_cp) {
@@ -449,7 +455,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
             }
           }
           // K = 64 lifted columns per instruction: 32 B of compressed weights, 64 B of activations per row
-          if (issue_mma) {
+          if (issue_mma && leader) {
             ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo, kDescHiA), desc(b_lo, kDescHiB), e_tmem, idesc, st != st_first ? 1u : 0u);
             ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo + 2, kDescHiA), desc(b_lo + 4, kDescHiB), e_tmem + 2, idesc, 1u);
             if (KB == 2 && full_stage) {
@@ -462,13 +468,13 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           // when they have completed): the MMAs queue ahead of the pipe, so the commit costs this
           // thread time the pipe does not wait for, and the refill is not held up by the next
           // stage's arrival.
-          ptx::tc_commit_pair(&bar_empty[slot], 3);
+          if (leader) ptx::tc_commit_pair(&bar_empty[slot], 3);
           SS_PF(pf_commit);
           if (slot == kRing - 1) phase ^= 1u;
           SS_PF(pf_peek);
           if (++st == st_end) {
             // the piece is complete: publish the accumulator
-            ptx::tc_commit_pair(&bar_acc_full[buf], 3);
+            if (leader) ptx::tc_commit_pair(&bar_acc_full[buf], 3);
             SS_PF(pf_commit);
             SS_TL(1, tl, 3);
             last_buf = buf;
@@ -482,7 +488,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
             buf = acc_it % T::kAccBufs;
             d_tmem = tmem_base + buf * NT;
             SS_TL(1, tl, 0);
-            if (!ptx::mbar_wait(&bar_acc_empty[buf], ((acc_it / T::kAccBufs) & 1u) ^ 1u, args.wait_ns)) { ok = false; more = false; break; }
+            if (!ptx::mbar_wait_warp(&bar_acc_empty[buf], ((acc_it / T::kAccBufs) & 1u) ^ 1u, args.wait_ns)) { ok = false; more = false; break; }
             SS_PF(pf_acc);
             SS_TL(1, tl, 1);
             ptx::tc_fence_after();
@@ -493,15 +499,16 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       SS_PF_STORE(12, pf_peek); SS_PF_STORE(13, static_cast<long long>(probe_stages));
       if (probe && ok && probe_stages > 0) {
         // the last tile's accumulator is complete when its barrier (this CTA's copy) flips
-        if (!ptx::mbar_wait(&bar_acc_full[last_buf], last_use & 1u, args.wait_ns)) ok = false;
-        args.probe[0] = static_cast<unsigned long long>(clock64() - probe_begin);
-        args.probe[1] = probe_stages;
+        if (!ptx::mbar_wait_warp(&bar_acc_full[last_buf], last_use & 1u, args.wait_ns)) ok = false;
+        if (leader) args.probe[0] = static_cast<unsigned long long>(clock64() - probe_begin);
+        if (leader) args.probe[1] = probe_stages;
       }
-      if (!ok) atomicOr(args.status, kStatusMmaTimeout);
+      if (!ok && leader) atomicOr(args.status, kStatusMmaTimeout);
     }
   } else if (warp == 2 + kPairEpiWarps) {
     // ------------------------------------------------------------------ metadata copier (rank 0 only)
-    if (meta_warp && lane == 0 && rank == 0) {
+    if (meta_warp && rank == 0) {
+      const bool leader = ptx::elect_one();
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (Walk<SPLIT> w(pair, num_pairs, tiles_ch2, num_tiles, num_st); w.valid && ok; w.advance()) {
@@ -510,11 +517,12 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           const int nkb = args.num_kb - kb0 < KB ? args.num_kb - kb0 : KB;
           // the stage's previous metadata is no longer read once its MMAs have completed, which
           // the producer has already waited for before refilling the stage
-          if (!ptx::mbar_wait(&bar_e[s], phase, args.wait_ns)) { ok = false; break; }
+          if (!ptx::mbar_wait_warp(&bar_e[s], phase, args.wait_ns)) { ok = false; break; }
           ptx::tc_fence_after();
           const uint32_t e_addr = ptx::smem_u32(smem + off_e + s * T::kEBytes);
           const uint32_t e_tmem = tmem_base + T::kMetaCol + s * T::kMetaColsPerStage;
-          if (KB == 2 && nkb == 2 && args.wide_cp) {
+          if (!leader) {
+          } else if (KB == 2 && nkb == 2 && args.wide_cp) {
             // both metadata blocks of the stage in one instruction: block h is the h-th 16-byte
             // column of a 128 x 32-byte matrix whose columns lie kEBlock bytes apart
             ptx::tc_cp_128x256b_pair(e_tmem, smem_desc(e_addr, T::kEBlock, 128, 0));
@@ -522,11 +530,11 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
             for (int h = 0; h < nkb; ++h)
               ptx::tc_cp_128x128b_pair(e_tmem + 4 * h, smem_desc(e_addr + h * T::kEBlock, 128, 128, 0));
           }
-          ptx::tc_commit_pair(&bar_full[s], 1);      // arrives (rank 0 only) when the copy has completed
+          if (leader) ptx::tc_commit_pair(&bar_full[s], 1);      // arrives (rank 0 only) when the copy has completed
           if (++s == static_cast<uint32_t>(kRing)) { s = 0; phase ^= 1u; }
         }
       }
-      if (!ok) atomicOr(args.status, kStatusMmaTimeout);
+      if (!ok && leader) atomicOr(args.status, kStatusMmaTimeout);
     }
   } else if constexpr (MODE == kOutBf16Tma || MODE == kOutBf16GateAdd || MODE == kOutBf16TmaPeers || MODE == kOutBf16TmaSplit) {
     // ------------------------------------------------------------------ epilogue, TMA stores
