@@ -311,7 +311,7 @@ int ss_device_status(void* stream, int32_t* status);
 /* The library reads its switches from the environment once, at first use (SS_TOKEN_TILE,
  * SS_WIDE_CP, SS_META_WARP, SS_STORE, SS_RESIDENT, SS_PDL, SS_SPLIT, SS_WAIT_NS); these two entries read and
  * change them afterwards, for tests and measurements.  No counterpart in the reference.  Names:
- * "token_tile" (0 = automatic, or 128/192/224/240/256), "wide_cp", "meta_warp" (-1 = automatic),
+ * "token_tile" (0 = automatic, or 128/192/224/240/256), "wide_cp", "meta_warp" (selects nothing any more),
  * "store" (1 = TMA-store epilogue), "resident" (weights-resident form), "pdl" (programmatic
  * dependent launch), "split" (schedule of the GEMM in which the clusters share the tiles x stages
  * evenly and a tile computed by several clusters is summed through device memory the library

@@ -46,7 +46,7 @@ constexpr unsigned long long kDefaultWaitNs = 2000000000ull;   // limit of every
 struct Options {
   int token_tile = 0;     // 0 = chosen per problem; 128 / 192 / 224 / 256 force a tile
   int wide_cp = 1;        // one tcgen05.cp.128x256b per stage instead of two 128x128b
-  int meta_warp = -1;     // -1 = by pipeline depth; 0 / 1 force the metadata-copy warp off / on
+  int meta_warp = -1;     // accepted and stored only: the MMA warp issues the metadata copies
   int store = 1;          // 1 = TMA-store epilogue where alignment allows, 0 = direct stores
   int resident = 1;       // weights-resident form where applicable
   int pdl = 1;            // programmatic dependent launch between front-end and GEMM

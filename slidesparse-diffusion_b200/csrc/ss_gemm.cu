@@ -9,7 +9,7 @@
 // and its columns are tokens, as in the reference (csrc/dualscale_sm80.cu:189-204).
 //
 // There is one kernel, sparse_gemm_pair_kernel (ss_gemm_pair.cuh): persistent clusters of two CTAs
-// (cta_group::2), warp-specialised into a TMA producer, an MMA issuer, a metadata copier and eight
+// (cta_group::2), warp-specialised into a TMA producer, an MMA and metadata-copy issuer and eight
 // epilogue warps per CTA, with two accumulators in TMEM so that the epilogue of one tile overlaps
 // the main loop of the next.  This file holds what the kernel needs around it: argument block,
 // descriptor helpers, the direct-store epilogue body, tile choice, tensor maps and the launch.
@@ -43,7 +43,6 @@ struct KernelArgs {
   int tiles_ch, tiles_tok, num_kb;
   uint32_t* status;
   int wide_cp;          // CTA-pair kernel: copy a stage's two metadata blocks with one tcgen05.cp
-  int meta_warp;        // CTA-pair kernel: a dedicated warp issues the metadata copies
   const __nv_bfloat16* gate;   // gated accumulation: BF16 [batches, n], rows gate_stride apart
   long long gate_stride;
   int rows_per_batch;
@@ -351,7 +350,6 @@ int launch_pair_t(const GemmArgs& a, DeviceInfo* dev, int tile_index, cudaStream
   k.gate_stride = a.gate_stride;
   k.rows_per_batch = static_cast<int>(a.rows_per_batch);
   k.wide_cp = opt.wide_cp;
-  k.meta_warp = opt.meta_warp >= 0 ? opt.meta_warp : (T::kStages >= 4 ? 1 : 0);
   k.res_stages = res_stages;
   k.peer_count = 0;
   k.wait_ns = a.wait_ns ? a.wait_ns : opt.wait_ns;

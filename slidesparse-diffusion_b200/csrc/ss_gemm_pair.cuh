@@ -12,14 +12,13 @@
 // issue, commits), now the round trip of the four-stage ring; see the diagnostics entry
 // ss_micro_pair_rate and the counters a -DSS_TIMELINE build keeps.
 //
-// Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer (rank 0 only; also allocates TMEM), warps
-// 2..9 epilogue (two per TMEM lane quadrant), warp 10 metadata copier (streaming form, rank 0).
+// Roles per CTA: warp 0 TMA producer, warp 1 MMA and metadata-copy issuer (rank 0 only; also allocates
+// TMEM), warps 2..9 epilogue (two per TMEM lane quadrant); warp 10 has none.
 //
 // Protocol (rank = %cluster_ctarank):
 //   full[s]      lives in rank 0 only.  Rank 0's producer posts the byte count of BOTH CTAs'
 //                loads; both producers issue their loads with the cta_group::2 form, which
-//                credits completion to rank 0's barrier; with a metadata warp its commit is the
-//                barrier's second arrival.
+//                credits completion to rank 0's barrier.
 //   empty[s]     one copy per CTA; the MMA thread (rank 0) commits with a 2-CTA multicast so
 //                both producers see the stage free at the same time.
 //   acc_full[b]  one copy per CTA, multicast commit; acc_empty[b] lives in rank 0 and counts the
@@ -33,10 +32,6 @@
 #endif
 constexpr int kPairEpiWarps = SS_PAIR_EPI_WARPS;       // 2 or 4 warps per TMEM lane quadrant
 constexpr int kPairSub = kPairEpiWarps / 4;            // warps sharing a quadrant take chunks sub, sub+kPairSub, ...
-// The last warp can issue the metadata copies (tcgen05.cp) so that the MMA thread, whose
-// cta_group::2 operations cost about 125 cycles each to issue, only issues MMAs and commits
-// (args.meta_warp).  It adds one barrier hop per stage, which pays with four or more pipeline
-// stages (token tiles up to 224: -6 % on 4096x3072->9216) and costs with three (256).
 constexpr int kPairThreads = 64 + 32 * kPairEpiWarps + 32;
 
 // Per-tile time stamps of the three roles of each cluster's rank-0 CTA, for builds made with
@@ -224,14 +219,11 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   uint64_t* bar_empty = bar_full + kBarStride;
   uint64_t* bar_acc_full = bar_empty + kBarStride;
   uint64_t* bar_acc_empty = bar_acc_full + T::kAccBufs;
-  // streaming form: metadata of a stage is in TMEM (rank 0).  Resident form: [0] metadata of the
-  // whole K extent is in TMEM (both CTAs), [1] resident operands have landed (rank 0)
+  // resident form: [0] metadata of the whole K extent is in TMEM (both CTAs), [1] resident operands
+  // have landed (rank 0)
   uint64_t* bar_meta = bar_acc_empty + T::kAccBufs;
-  // streaming form: the metadata of a stage has landed in shared memory (rank 0).  It has a barrier
-  // of its own so that its copy into TMEM runs while the stage's weights and activations still land.
-  uint64_t* bar_e = bar_meta + kBarStride;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_e + kBarStride);
-  static_assert((5 * kBarStride + 2 * T::kAccBufs) * 8 + 8 <= T::kBarBytes, "barrier block");
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_meta + 2);
+  static_assert((2 * kBarStride + 2 * T::kAccBufs + 2) * 8 + 8 <= T::kBarBytes, "barrier block");
   static_assert(!RES || T::kAccBufs == 2, "resident form assumes two accumulators");
   static_assert(!(T::kHalfTail && MODE == kOutBf16TmaPeers), "the tensor-parallel stores take whole chunks only");
 
@@ -240,7 +232,6 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int tiles_ch2 = (args.tiles_ch + 1) >> 1;            // tiles of 256 channels
   const int num_tiles = tiles_ch2 * args.tiles_tok;
-  const bool meta_warp = !RES && args.meta_warp != 0;
   // Tile sequence of this cluster: pair, pair + num_pairs, ...; tile = token tile * tiles_ch2 +
   // channel tile.  The resident form is launched with a cluster count that is a multiple of
   // tiles_ch2, so every tile of a cluster has the same channel tile (tile % tiles_ch2).
@@ -248,13 +239,9 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kBarStride; ++s) {
-      // a stage is ready when its operands have landed (the producer's arrival + the bytes) and, with
-      // a metadata warp, when its metadata has been copied into TMEM (that warp's commit): one
-      // barrier, so that the MMA thread polls once per stage
-      ptx::mbar_init(&bar_full[s], meta_warp ? 2 : 1);
+      ptx::mbar_init(&bar_full[s], 1);      // the producer's arrival + the bytes of both CTAs
       ptx::mbar_init(&bar_empty[s], 1);
-      ptx::mbar_init(&bar_meta[s], 1);
-      ptx::mbar_init(&bar_e[s], 1);
+      if (RES && s < 2) ptx::mbar_init(&bar_meta[s], 1);
     }
     for (int b = 0; b < T::kAccBufs; ++b) {
       ptx::mbar_init(&bar_acc_full[b], 1);
@@ -299,7 +286,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       bool ok = true;
       long long pf_wait = 0, pf_arm = 0, pf_a = 0, pf_b = 0, pf_e = 0;
       (void)pf_wait; (void)pf_arm; (void)pf_a; (void)pf_b; (void)pf_e;
-      constexpr uint32_t kStageTx = 2u * (RES ? T::kBBytes : T::kABytes + T::kBBytes);   // both CTAs' bytes
+      constexpr uint32_t kStageTx = 2u * (RES ? T::kBBytes : T::kStageBytes);   // both CTAs' bytes
       if constexpr (RES) {
         // the weights do not depend on the preceding kernel: fetch the resident operands first
         if (tile_first < num_tiles) {
@@ -324,14 +311,10 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           if (!ptx::mbar_wait_warp(&bar_empty[s], phase ^ 1u, args.wait_ns)) { ok = false; break; }
           SS_PF(pf_wait);
           if (leader) {
-            if (rank == 0) {
-              if constexpr (!RES) ptx::mbar_arrive_expect_tx(&bar_e[s], 2u * T::kEBytes);
-              ptx::mbar_arrive_expect_tx(&bar_full[s], kStageTx);
-            }
+            if (rank == 0) ptx::mbar_arrive_expect_tx(&bar_full[s], kStageTx);
             SS_PF(pf_arm);
             if constexpr (!RES) {
-              // the metadata first: it is small, and its copy into TMEM can start while the rest lands
-              ptx::tma_load_3d_pair(smem + off_e + s * T::kEBytes, &map_e, &bar_e[s], 0, ch0 >> 5, st * KB);
+              ptx::tma_load_3d_pair(smem + off_e + s * T::kEBytes, &map_e, &bar_full[s], 0, ch0 >> 5, st * KB);
               SS_PF(pf_e);
             }
             ptx::tma_load_3d_pair(smem + off_b + s * T::kBBytes, &map_b, &bar_full[s], 0, tok0, st * KB);
@@ -361,18 +344,14 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           for (uint32_t f = 0; f < static_cast<uint32_t>(kRing) && f < issued; ++f) {
             const uint32_t fills = (issued - f + kRing - 1) / kRing;
             ptx::mbar_wait(&bar_full[f], (fills - 1) & 1u, limit);
-            if constexpr (!RES) ptx::mbar_wait(&bar_e[f], (fills - 1) & 1u, limit);
           }
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (rank 0 only)
-    // The tensor pipe queues next to nothing: an MMA is accepted when the one before it is nearly
-    // done, so whatever else this thread executes between two MMAs (address arithmetic, barrier
-    // polls, commits) is time the pipe stands idle.  The ring is therefore unrolled with the stage
-    // slot as a compile-time constant: every shared-memory descriptor is one add away from a
-    // value computed before the loop, and a stage costs four MMAs, one commit and one barrier poll.
+    // A rolled loop: one copy of the stage's code, short enough to stay in the instruction caches that
+    // eleven warps in four different loops share.
     if (rank == 0) {
       const bool leader = ptx::elect_one();
       constexpr uint32_t idesc = (1u << 2) | (2u << 4) | (1u << 7) | (1u << 10) |
@@ -384,9 +363,10 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       constexpr uint32_t kDescHiB = (1024u >> 4) | (1u << 14) | (2u << 29);
       const uint32_t a_lo0 = ((ptx::smem_u32(smem + off_a) & 0x3ffffu) >> 4) | (1u << 16);
       const uint32_t b_lo0 = ((ptx::smem_u32(smem + off_b) & 0x3ffffu) >> 4) | (1u << 16);
+      const uint32_t e_addr0 = ptx::smem_u32(smem + off_e);
       auto desc = [](uint32_t lo, uint32_t hi) { return (static_cast<uint64_t>(hi) << 32) | lo; };
       const bool odd_tail = (args.num_kb % KB) != 0;       // the last stage of a tile holds one block only
-      uint32_t phase = 0, acc_it = 0;
+      uint32_t slot = 0, phase = 0, acc_it = 0;
       bool ok = true;
       // diagnostics (ss_micro_pair_rate): cluster 0 reports the cycles its tile loop took; bit 0 of
       // args.debug leaves the MMAs out (commits only), so that the operand feed is timed alone
@@ -396,14 +376,12 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       uint32_t probe_stages = 0, last_buf = 0, last_use = 0, tl = 0;
       long long pf_acc = 0, pf_ready = 0, pf_mma = 0, pf_commit = 0, pf_peek = 0;
       (void)pf_acc; (void)pf_ready; (void)pf_mma; (void)pf_commit; (void)pf_peek;
-      Walk<SPLIT> w(pair, num_pairs, tiles_ch2, num_tiles, num_st);
-      bool more = w.valid;
       if constexpr (RES) {
         // once per cluster: metadata of the whole K extent from its staging area into TMEM
-        if (more) {
+        if (tile_first < num_tiles) {
           if (!ptx::mbar_wait_warp(&bar_meta[1], 0, args.wait_ns)) ok = false;
           ptx::tc_fence_after();
-          const uint32_t e_addr = ptx::smem_u32(smem + off_e);
+          const uint32_t e_addr = e_addr0;
           const uint32_t e_tmem = tmem_base + T::kMetaCol;
           for (int kb = 0; kb < args.num_kb && ok && leader; kb += 2) {
             if (kb + 1 < args.num_kb && args.wide_cp)
@@ -416,84 +394,63 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         }
       }
       if (probe) probe_begin = clock64();
-      int st = w.s0, st_first = w.s0, st_end = w.s1;      // the current piece's stages
-      uint32_t buf = 0, d_tmem = tmem_base;
-      if (more && ok) {
+      for (Walk<SPLIT> w(pair, num_pairs, tiles_ch2, num_tiles, num_st); w.valid && ok; w.advance(), ++acc_it, ++tl) {
+        const uint32_t buf = acc_it % T::kAccBufs, d_tmem = tmem_base + buf * NT;
+        SS_PF_BEGIN();
         SS_TL(1, tl, 0);
-        if (!ptx::mbar_wait_warp(&bar_acc_empty[0], 1u, args.wait_ns)) ok = false;
+        if (!ptx::mbar_wait_warp(&bar_acc_empty[buf], ((acc_it / T::kAccBufs) & 1u) ^ 1u, args.wait_ns)) { ok = false; break; }
+        SS_PF(pf_acc);
         SS_TL(1, tl, 1);
         ptx::tc_fence_after();
-      }
-      while (more && ok) {
-#pragma unroll
-        for (int slot = 0; slot < kRing; ++slot) {
-          SS_PF_BEGIN();
-          if (!ptx::mbar_wait_warp(&bar_full[slot], phase, args.wait_ns)) { ok = false; more = false; break; }
-          if constexpr (!RES) {
-            // without a metadata warp this thread copies the stage's metadata itself (below)
-            if (!meta_warp && !ptx::mbar_wait_warp(&bar_e[slot], phase, args.wait_ns)) { ok = false; more = false; break; }
-          }
+#pragma unroll 1
+        for (int st = w.s0; st < w.s1; ++st) {
+          if (!ptx::mbar_wait_warp(&bar_full[slot], phase, args.wait_ns)) { ok = false; break; }
           SS_PF(pf_ready);
-          if (st == st_first) SS_TL(1, tl, 2);
+          if (st == w.s0) SS_TL(1, tl, 2);
           ++probe_stages;
-          ptx::tc_fence_after();
           // resident form: weights and metadata are indexed by the K position, not by the ring slot
-          const uint32_t a_lo = a_lo0 + static_cast<uint32_t>(RES ? st : slot) * (T::kABytes >> 4);
-          const uint32_t b_lo = b_lo0 + static_cast<uint32_t>(slot) * (T::kBBytes >> 4);
-          const uint32_t e_tmem = tmem_base + T::kMetaCol + static_cast<uint32_t>(RES ? st : slot) * T::kMetaColsPerStage;
+          const uint32_t a_at = RES ? static_cast<uint32_t>(st) : slot;
+          const uint32_t a_lo = a_lo0 + a_at * (T::kABytes >> 4);
+          const uint32_t b_lo = b_lo0 + slot * (T::kBBytes >> 4);
+          const uint32_t e_tmem = tmem_base + T::kMetaCol + a_at * T::kMetaColsPerStage;
           const bool full_stage = !(odd_tail && st == num_st - 1);
-          if (!RES && !meta_warp && leader) {
-            // no metadata warp (three pipeline stages): this thread copies the stage's metadata itself
-            const uint32_t e_addr = ptx::smem_u32(smem + off_e) + slot * T::kEBytes;
-            if (KB == 2 && full_stage && args.wide_cp) {
-              // both metadata blocks of the stage in one instruction: block h is the h-th 16-byte
-              // column of a 128 x 32-byte matrix whose columns lie kEBlock bytes apart
-              ptx::tc_cp_128x256b_pair(e_tmem, smem_desc(e_addr, T::kEBlock, 128, 0));
-            } else {
-              for (int h = 0; h < (full_stage ? KB : 1); ++h)
-                ptx::tc_cp_128x128b_pair(e_tmem + 4 * h, smem_desc(e_addr + h * T::kEBlock, 128, 128, 0));
+          if (leader) {
+            if constexpr (!RES) {
+              // The stage's metadata, from shared memory into TMEM.  Copies and MMAs of one thread
+              // execute in order, so nothing has to be waited for in between; with a warp of its own
+              // for the copies, their commit and its barrier were on every stage's way.
+              const uint32_t e_addr = e_addr0 + slot * T::kEBytes;
+              if (KB == 2 && full_stage && args.wide_cp) {
+                // both metadata blocks of the stage in one instruction: block h is the h-th 16-byte
+                // column of a 128 x 32-byte matrix whose columns lie kEBlock bytes apart
+                ptx::tc_cp_128x256b_pair(e_tmem, smem_desc(e_addr, T::kEBlock, 128, 0));
+              } else {
+                for (int h = 0; h < (full_stage ? KB : 1); ++h)
+                  ptx::tc_cp_128x128b_pair(e_tmem + 4 * h, smem_desc(e_addr + h * T::kEBlock, 128, 128, 0));
+              }
             }
-          }
-          // K = 64 lifted columns per instruction: 32 B of compressed weights, 64 B of activations per row
-          if (issue_mma && leader) {
-            ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo, kDescHiA), desc(b_lo, kDescHiB), e_tmem, idesc, st != st_first ? 1u : 0u);
-            ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo + 2, kDescHiA), desc(b_lo + 4, kDescHiB), e_tmem + 2, idesc, 1u);
-            if (KB == 2 && full_stage) {
-              ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo + 4, kDescHiA), desc(b_lo + (T::kBBlock >> 4), kDescHiB), e_tmem + 4, idesc, 1u);
-              ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo + 6, kDescHiA), desc(b_lo + (T::kBBlock >> 4) + 4, kDescHiB), e_tmem + 6, idesc, 1u);
+            // K = 64 lifted columns per instruction: 32 B of compressed weights, 64 B of activations per row
+            if (issue_mma) {
+              ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo, kDescHiA), desc(b_lo, kDescHiB), e_tmem, idesc, st != w.s0 ? 1u : 0u);
+              ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo + 2, kDescHiA), desc(b_lo + 4, kDescHiB), e_tmem + 2, idesc, 1u);
+              if (KB == 2 && full_stage) {
+                ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo + 4, kDescHiA), desc(b_lo + (T::kBBlock >> 4), kDescHiB), e_tmem + 4, idesc, 1u);
+                ptx::tc_mma_sp_i8_pair(d_tmem, desc(a_lo + 6, kDescHiA), desc(b_lo + (T::kBBlock >> 4) + 4, kDescHiB), e_tmem + 6, idesc, 1u);
+              }
             }
-          }
-          SS_PF(pf_mma);
-          // The stage goes back to the producers as soon as its MMAs are queued (the arrival happens
-          // when they have completed): the MMAs queue ahead of the pipe, so the commit costs this
-          // thread time the pipe does not wait for, and the refill is not held up by the next
-          // stage's arrival.
-          if (leader) ptx::tc_commit_pair(&bar_empty[slot], 3);
-          SS_PF(pf_commit);
-          if (slot == kRing - 1) phase ^= 1u;
-          SS_PF(pf_peek);
-          if (++st == st_end) {
-            // the piece is complete: publish the accumulator
-            if (leader) ptx::tc_commit_pair(&bar_acc_full[buf], 3);
+            SS_PF(pf_mma);
+            // the stage goes back to the producers when its MMAs have completed
+            ptx::tc_commit_pair(&bar_empty[slot], 3);
+            // and with the piece's last stage its accumulator is complete
+            if (st + 1 == w.s1) ptx::tc_commit_pair(&bar_acc_full[buf], 3);
             SS_PF(pf_commit);
-            SS_TL(1, tl, 3);
-            last_buf = buf;
-            last_use = acc_it / T::kAccBufs;
-            w.advance();
-            ++acc_it;
-            ++tl;
-            if (!w.valid) { more = false; break; }
-            st = st_first = w.s0;
-            st_end = w.s1;
-            buf = acc_it % T::kAccBufs;
-            d_tmem = tmem_base + buf * NT;
-            SS_TL(1, tl, 0);
-            if (!ptx::mbar_wait_warp(&bar_acc_empty[buf], ((acc_it / T::kAccBufs) & 1u) ^ 1u, args.wait_ns)) { ok = false; more = false; break; }
-            SS_PF(pf_acc);
-            SS_TL(1, tl, 1);
-            ptx::tc_fence_after();
           }
+          __syncwarp();
+          if (++slot == static_cast<uint32_t>(kRing)) { slot = 0; phase ^= 1u; }
         }
+        SS_TL(1, tl, 3);
+        last_buf = buf;
+        last_use = acc_it / T::kAccBufs;
       }
       SS_PF_STORE(8, pf_acc); SS_PF_STORE(9, pf_ready); SS_PF_STORE(10, pf_mma); SS_PF_STORE(11, pf_commit);
       SS_PF_STORE(12, pf_peek); SS_PF_STORE(13, static_cast<long long>(probe_stages));
@@ -506,36 +463,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       if (!ok && leader) atomicOr(args.status, kStatusMmaTimeout);
     }
   } else if (warp == 2 + kPairEpiWarps) {
-    // ------------------------------------------------------------------ metadata copier (rank 0 only)
-    if (meta_warp && rank == 0) {
-      const bool leader = ptx::elect_one();
-      uint32_t s = 0, phase = 0;
-      bool ok = true;
-      for (Walk<SPLIT> w(pair, num_pairs, tiles_ch2, num_tiles, num_st); w.valid && ok; w.advance()) {
-        for (int st = w.s0; st < w.s1; ++st) {
-          const int kb0 = st * KB;
-          const int nkb = args.num_kb - kb0 < KB ? args.num_kb - kb0 : KB;
-          // the stage's previous metadata is no longer read once its MMAs have completed, which
-          // the producer has already waited for before refilling the stage
-          if (!ptx::mbar_wait_warp(&bar_e[s], phase, args.wait_ns)) { ok = false; break; }
-          ptx::tc_fence_after();
-          const uint32_t e_addr = ptx::smem_u32(smem + off_e + s * T::kEBytes);
-          const uint32_t e_tmem = tmem_base + T::kMetaCol + s * T::kMetaColsPerStage;
-          if (!leader) {
-          } else if (KB == 2 && nkb == 2 && args.wide_cp) {
-            // both metadata blocks of the stage in one instruction: block h is the h-th 16-byte
-            // column of a 128 x 32-byte matrix whose columns lie kEBlock bytes apart
-            ptx::tc_cp_128x256b_pair(e_tmem, smem_desc(e_addr, T::kEBlock, 128, 0));
-          } else {
-            for (int h = 0; h < nkb; ++h)
-              ptx::tc_cp_128x128b_pair(e_tmem + 4 * h, smem_desc(e_addr + h * T::kEBlock, 128, 128, 0));
-          }
-          if (leader) ptx::tc_commit_pair(&bar_full[s], 1);      // arrives (rank 0 only) when the copy has completed
-          if (++s == static_cast<uint32_t>(kRing)) { s = 0; phase ^= 1u; }
-        }
-      }
-      if (!ok && leader) atomicOr(args.status, kStatusMmaTimeout);
-    }
+    // no role: it arrives at the closing barriers
   } else if constexpr (MODE == kOutBf16Tma || MODE == kOutBf16GateAdd || MODE == kOutBf16TmaPeers || MODE == kOutBf16TmaSplit) {
     // ------------------------------------------------------------------ epilogue, TMA stores
     constexpr bool GATED = MODE == kOutBf16GateAdd;
