@@ -300,6 +300,16 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t saddr, uint32_t a, ui
                ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d)
                : "memory");
 }
+// The load with the same addresses and the same distribution over the threads.
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t saddr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(saddr)
+               : "memory");
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t saddr, const uint4& v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 // Programmatic dependent launch: a kernel launched with programmatic stream serialization may
 // start once every CTA of the preceding kernel has called grid_dep_launch (or exited); it must
 // call grid_dep_wait before touching anything that kernel writes.  Both are no-ops otherwise.

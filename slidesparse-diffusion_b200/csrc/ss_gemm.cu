@@ -135,7 +135,7 @@ struct MapKeyEq {
 constexpr size_t kMapCacheLimit = 8192;   // descriptors kept; the cache starts over beyond this
 
 // kernel variants: token tile x output mode x resident form
-constexpr int kTileCount = 5, kModeCount = 7;
+constexpr int kTileCount = 5, kModeCount = 8;
 struct DeviceInfo {
   int sms = 0;
   std::atomic<bool> configured[kTileCount][kModeCount][2];
@@ -391,7 +391,7 @@ int launch_pair_t(const GemmArgs& a, DeviceInfo* dev, int tile_index, cudaStream
   }
   map_out = map_a;         // unused by the direct-store epilogues
   map_out_tail = map_a;
-  if constexpr (MODE == kOutBf16Tma || MODE == kOutBf16GateAdd || MODE == kOutBf16TmaSplit) {
+  if constexpr (MODE == kOutBf16Tma || MODE == kOutBf16GateAdd || MODE == kOutBf16TmaSplit || MODE == kOutBf16TmaAddend) {
     // out[m, n] BF16, row pitch out_stride: one 32-channel x 32-token box per epilogue warp and chunk;
     // the epilogue writes its 64-byte rows with the 16-byte pieces XOR-swizzled (bank-conflict-free stmatrix)
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(a.n), static_cast<cuuint64_t>(a.m)};
@@ -481,8 +481,13 @@ template <int NT, int KB>
 int launch_pair_nt(const GemmArgs& a, DeviceInfo* dev, int tile_index, cudaStream_t stream, int res_stages = 0, bool split = false) {
   if (split) return launch_pair_t<NT, KB, kOutBf16TmaSplit>(a, dev, tile_index, stream);
   if (a.int32_out) return launch_pair_t<NT, KB, kOutInt32>(a, dev, tile_index, stream);
-  if (a.addend) return launch_pair_t<NT, KB, kOutBf16Addend>(a, dev, tile_index, stream);
   const bool aligned = tma_store_ok(a);
+  if (a.addend) {
+    // 16-byte reads of the addend need what TMA stores need of the output
+    const bool rows16 = (reinterpret_cast<uintptr_t>(a.addend) & 15) == 0 && a.addend_stride % 8 == 0;
+    if (aligned && rows16 && options().store == 1) return launch_pair_t<NT, KB, kOutBf16TmaAddend>(a, dev, tile_index, stream);
+    return launch_pair_t<NT, KB, kOutBf16Addend>(a, dev, tile_index, stream);
+  }
   if constexpr (KB == 2 && (NT == 192 || NT == 224)) {
     if (res_stages > 0 && aligned) {
       if (a.gate) return launch_pair_t<NT, KB, kOutBf16GateAdd, true>(a, dev, tile_index, stream, res_stages);

@@ -157,6 +157,7 @@ enum : int {
   kOutBf16GateAdd = 4, // as kOutBf16Tma, but out += bf16(gate[batch, channel] * y) by TMA reduction
   kOutBf16TmaPeers = 5, // as kOutBf16Tma, but every tile is stored to several destinations (peer GPUs)
   kOutBf16TmaSplit = 6, // as kOutBf16Tma with the split schedule (see Walk): tiles may be shared by clusters
+  kOutBf16TmaAddend = 7, // as kOutBf16Tma with an addend (16-byte aligned rows)
 };
 
 // Destination tensor maps of the tensor-parallel form; the other forms pass an empty struct.
@@ -251,7 +252,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     ptx::prefetch_tensormap(&map_a);
     ptx::prefetch_tensormap(&map_b);
     ptx::prefetch_tensormap(&map_e);
-    if constexpr (MODE == kOutBf16Tma || MODE == kOutBf16GateAdd || MODE == kOutBf16TmaSplit) {
+    if constexpr (MODE == kOutBf16Tma || MODE == kOutBf16GateAdd || MODE == kOutBf16TmaSplit || MODE == kOutBf16TmaAddend) {
       ptx::prefetch_tensormap(&map_out);
       if constexpr (T::kHalfTail) ptx::prefetch_tensormap(&map_out_tail);
     }
@@ -464,9 +465,10 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     }
   } else if (warp == 2 + kPairEpiWarps) {
     // no role: it arrives at the closing barriers
-  } else if constexpr (MODE == kOutBf16Tma || MODE == kOutBf16GateAdd || MODE == kOutBf16TmaPeers || MODE == kOutBf16TmaSplit) {
+  } else if constexpr (MODE == kOutBf16Tma || MODE == kOutBf16GateAdd || MODE == kOutBf16TmaPeers || MODE == kOutBf16TmaSplit ||
+                       MODE == kOutBf16TmaAddend) {
     // ------------------------------------------------------------------ epilogue, TMA stores
-    constexpr bool GATED = MODE == kOutBf16GateAdd;
+    constexpr bool GATED = MODE == kOutBf16GateAdd, ADDEND = MODE == kOutBf16TmaAddend;
     // The accumulator is channel-major in TMEM (lane = channel, column = token) and the output is
     // token-major.  tcgen05.ld in the 16x256b fragment layout hands each thread two adjacent
     // tokens of one channel per register pair, which is exactly what stmatrix.trans needs to
@@ -551,6 +553,24 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       chunks = chunks < T::kChunks ? chunks : T::kChunks;
       const int mine = chunks > half ? (chunks - half + kPairSub - 1) / kPairSub : 0;
       uint32_t f[2][32];
+      // Addend form: a chunk's 32 x 32 piece of the addend is read in 64-byte rows (four lanes each) one
+      // chunk ahead, the first one while the tile's MMAs still run, and passes through the staging tile
+      // into the distribution of the accumulator.  Read from the accumulator's distribution directly
+      // (one channel per lane, a load and a 2-byte store per token) 1536 x 12288 -> 3072 took 97 us; 40
+      // without an addend.
+      uint4 ad[ADDEND ? 4 : 1];
+      auto load_addend = [&](int c) {
+#pragma unroll
+        for (int j = 0; j < (ADDEND ? 4 : 0); ++j) {
+          const int tok = tok0 + c * 32 + 8 * j + (lane >> 2), ch = ch_w + 8 * (lane & 3);
+          ad[j] = make_uint4(0u, 0u, 0u, 0u);
+          if (tok < args.m && ch < args.n)
+            ad[j] = __ldg(reinterpret_cast<const uint4*>(args.addend + static_cast<long long>(tok) * args.addend_stride + ch));
+        }
+      };
+      if constexpr (ADDEND) {
+        if (mine > 0) load_addend(half);
+      }
       // split schedule: this warp's chunk i of a slab into registers
       auto fetch = [&](uint32_t (&r)[32], const uint4* src, int i) {
 #pragma unroll
@@ -629,11 +649,24 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         // rows are 64 bytes (32 channels) with the 16-byte pieces XOR-swizzled as TMA's 64B mode expects
         const int mi = lane >> 3;
         const uint32_t stage_addr = ptx::smem_u32(stage);
+        if constexpr (ADDEND) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int row = 8 * j + (lane >> 2);
+            ptx::st_shared_v4(stage_addr + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4), ad[j]);
+          }
+          if (c + kPairSub < chunks) load_addend(c + kPairSub);
+          __syncwarp();
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
 #pragma unroll
           for (int gp = 0; gp < 2; ++gp) {
-            uint32_t packed[4];
+            const int tok = 8 * (2 * gp + (mi >> 1)) + (lane & 7);
+            const int cg = 2 * h + (mi & 1);
+            const uint32_t block = stage_addr + tok * 64 + ((cg ^ ((tok >> 1) & 3)) << 4);
+            uint32_t packed[4], addend[4];
+            if constexpr (ADDEND) ptx::ldmatrix_x4_trans(block, addend);
 #pragma unroll
             for (int gi = 0; gi < 2; ++gi) {
               const int g = 2 * gp + gi;
@@ -648,14 +681,15 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                                                __int2float_rn(static_cast<int32_t>(r[2 * ab + 1])));
                 float2 y = __ffma2_rn(acc, __fmul2_rn(s, make_float2(w, w)), make_float2(b, b));
                 if constexpr (GATED) y = __fmul2_rn(make_float2(gate[2 * h + ab], gate[2 * h + ab]), y);
+                if constexpr (ADDEND) {
+                  const uint32_t t = addend[2 * gi + ab];
+                  y = make_float2(__fadd_rn(y.x, __uint_as_float(t << 16)), __fadd_rn(y.y, __uint_as_float(t & 0xffff0000u)));
+                }
                 const __nv_bfloat162 p = __floats2bfloat162_rn(y.x, y.y);   // low half = even token
                 packed[2 * gi + ab] = *reinterpret_cast<const uint32_t*>(&p);
               }
             }
-            const int tok = 8 * (2 * gp + (mi >> 1)) + (lane & 7);
-            const int cg = 2 * h + (mi & 1);
-            ptx::stmatrix_x4_trans(stage_addr + tok * 64 + ((cg ^ ((tok >> 1) & 3)) << 4),
-                                   packed[0], packed[1], packed[2], packed[3]);
+            ptx::stmatrix_x4_trans(block, packed[0], packed[1], packed[2], packed[3]);
           }
         }
         SS_PF(pe_math);
