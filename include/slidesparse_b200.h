@@ -103,7 +103,7 @@ int ss_obs_trailing(float* w, int64_t rows, int64_t columns, int64_t start, int6
 /* Export of compress (diffusion_research/reconstruction.py:117-127): qweight = clamp(rint(w/scale))
  * with the selected zeros forced to 0.  status (device int32[1], zeroed by the caller) gets bit 0
  * if check_grid and some qweight*scale differs from w, bit 1 if a complete group of `group`
- * columns holds more than group-2 nonzeros. */
+ * columns holds more than group-2 nonzeros, bit 2 if w holds a non-finite value. */
 int ss_obs_finish(const float* w, const float* scales, const uint8_t* zeros, int64_t rows,
                   int64_t columns, int group, int check_grid, int8_t* qweight, int32_t* status,
                   void* stream);

@@ -310,6 +310,19 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t saddr, uint32_t (&r)[
 __device__ __forceinline__ void st_shared_v4(uint32_t saddr, const uint4& v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
+// Asynchronous copies from global to shared memory, 4 or 16 bytes a thread (both addresses aligned to
+// the size); the 16-byte form copies `bytes` (0 or 16) of them and fills the rest with zeros.
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Programmatic dependent launch: a kernel launched with programmatic stream serialization may
 // start once every CTA of the preceding kernel has called grid_dep_launch (or exited); it must
 // call grid_dep_wait before touching anything that kernel writes.  Both are no-ops otherwise.

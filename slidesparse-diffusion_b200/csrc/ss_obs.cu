@@ -3,218 +3,379 @@
 // (reference: sdacc/diffusion_research/reconstruction.py:55-133, `compress`).
 //
 // Output rows are independent and all share one curvature factor, so a column block is processed
-// by eight lanes per row: the row's slice lives in shared memory next to the block's factor tile,
-// the lanes walk the columns in order (selection at each group start, rounding, error, rank-one
-// update of the columns still open) and the errors of the block are then applied to all later
-// columns by an fp32 GEMM with a fixed summation order.  Every floating-point operation is a
-// separately rounded IEEE operation in the order the reference's tensor expressions apply them
-// (the GEMM accumulates with fused multiply-adds in increasing k), which the CPU oracle repeats.
+// by four lanes per row: the row's slice lives in shared memory next to the block's factor tile,
+// the lanes walk the groups in order (selection at the group's start, then rounding, error and
+// update column by column inside the group, then the group's errors on the columns still open) and
+// the errors of the block are applied to all later columns by an fp32 GEMM with a fixed summation
+// order.  Every floating-point result is that of a separately rounded IEEE operation in the order
+// the reference's tensor expressions apply them (the GEMM accumulates with fused multiply-adds in
+// increasing k), which the CPU oracle repeats.
 #include "ss_common.cuh"
 
 namespace ss {
 namespace {
 
-constexpr int kObsWarps = 16;        // warps per CTA
-constexpr int kLanesPerRow = 8;      // a quarter of a warp walks one row (the widest group has 8 columns)
-constexpr int kRowsPerCta = kObsWarps * 32 / kLanesPerRow;
+constexpr int kLanesPerRow = 4;
+constexpr int kRowsPerWarp = 32 / kLanesPerRow;
+constexpr int kObsMaxRows = 64;      // rows a CTA walks at a time, at most
+constexpr int kObsMaxWidth = 225;    // widest column block
+
+// a / b, correctly rounded, from y = RN(1 / b): two residual corrections of the product a * y.  The
+// first makes the quotient faithful, after which the second gives the rounded one (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", 1990; needs b, y, the
+// quotient and the residuals to stay clear of overflow and underflow, which the callers' ranges see to).
+__device__ __forceinline__ float quotient(float a, float b, float y) {
+  float q = __fmul_rn(a, y);
+  q = __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
 
 __device__ __forceinline__ float round_to_grid(float v, float s) {
   // torch.round(v / s).clamp(-128, 127): round half to even
   return fminf(127.f, fmaxf(-128.f, rintf(__fdiv_rn(v, s))));
 }
 
-// Lowest (score, column) pair of the 8 lanes that walk one row; ties go to the lower column.
-__device__ __forceinline__ int argmin8(float score, int g) {
-#pragma unroll
-  for (int d = 4; d; d >>= 1) {
-    const float other = __shfl_xor_sync(0xffffffffu, score, d);
-    const int other_g = __shfl_xor_sync(0xffffffffu, g, d);
-    if (other < score || (other == score && other_g < g)) { score = other; g = other_g; }
-  }
-  return g;
-}
+// Ranges in which quotient() is exact: divisors 2^-15 .. 2^15 (their squares 2^-30 .. 2^30), scales
+// 2^-60 .. 2^60, dividends 2^-90 .. 2^60.  Outside (and for NaN) the IEEE division runs.
+__device__ __forceinline__ bool within(float v, float lo, float hi) { return fabsf(v) >= lo && fabsf(v) <= hi; }
 
-// One column block [start, start+width).  Eight lanes walk one row: the scalar chain of a column
-// (rounding, error) is repeated by those eight lanes only and the rank-one update of the columns
-// still open is shared between them.  Shared memory: the upper triangle of the block's factor
-// tile, row after row (row i starts at i*width - i*(i-1)/2 and holds columns i..width-1), then per
-// row two float rows (open values, which become the finalised ones, and errors) and one byte row
-// (selected zeros).
-__global__ void __launch_bounds__(kObsWarps * 32)
+__host__ __device__ __forceinline__ int obs_pitch(int width) {
+  // floats between two rows' open values: 16 (mod 32), so that the 16-byte accesses of two rows'
+  // lanes fall into different banks
+  return (width + 47) / 32 * 32 - 16;
+}
+// Factor tile: the upper triangle row after row, row i from column i rounded down to 4 up to the
+// width rounded up to 4.  This is where column j of row i lies, less j.
+__host__ __device__ __forceinline__ int obs_row(int i, int width) {
+  const int wp = (width + 3) & ~3, a = i >> 2;
+  return 4 * a * wp - 8 * a * (a - 1) + (i & 3) * (wp - 4 * a) - 4 * a;
+}
+__host__ __device__ __forceinline__ int obs_tile_floats(int width) { return obs_row(width, width) + (width & ~3); }
+
+// One column block [start, start+width).  Bound by the dependent chain of a column.  All four lanes of
+// a row walk it together in registers, a group at a time (the reciprocals of the divisors are made
+// once, which turns a division into five dependent multiply-adds), and they share the update of the
+// columns still open, group by group, 16 bytes at a time in the packed form of two.  Eight lanes per row,
+// a division in each step of the chain and an update of all open columns per column: 161 us per block of
+// 192 columns, 9216 rows; now 101 us.
+// Shared memory: factor tile, three reciprocal rows, then per row two float rows (open values, which
+// become the finalised ones, and errors), then a byte per group and row (its selected zeros).
+template <int G>
+__global__ void __launch_bounds__(kObsMaxRows * kLanesPerRow, 1)
 obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start, int width, int rows_per_cta,
-                 const float* __restrict__ upper, const float* __restrict__ scales, int group, int joint,
+                 const float* __restrict__ upper, const float* __restrict__ scales, int joint, float minus_zero,
                  uint8_t* __restrict__ zeros, float* __restrict__ errors, float* __restrict__ losses) {
   extern __shared__ __align__(16) unsigned char smem[];
-  float* tri = reinterpret_cast<float*>(smem);
-  const int tri_size = (width * (width + 1) / 2 + 3) & ~3;      // keeps the rows behind it 16-byte aligned
-  const int lane = threadIdx.x & 31, sl = lane & (kLanesPerRow - 1);
-  const int slot = threadIdx.x / kLanesPerRow;
-  float* open = tri + tri_size + slot * 2 * width;
-  float* err = open + width;
-  uint8_t* chosen = reinterpret_cast<uint8_t*>(tri + tri_size + kRowsPerCta * 2 * width) + slot * width;
+  float* tile = reinterpret_cast<float*>(smem);
+  const int wp = (width + 3) & ~3, pitch = obs_pitch(width), groups = (width + G - 1) / G;
+  float* recip = tile + obs_tile_floats(width);              // of the diagonal
+  float* square = recip + wp;                                // diagonal squared, and its reciprocal
+  float* square_recip = square + wp;
+  float* open_all = square_recip + wp;
+  float* err_all = open_all + rows_per_cta * pitch;
+  uint8_t* chosen_all = reinterpret_cast<uint8_t*>(err_all + rows_per_cta * pitch);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sl = lane & (kLanesPerRow - 1);
+  const int slot = threadIdx.x / kLanesPerRow, warps = blockDim.x >> 5;
 
-  for (int i = threadIdx.x; i < width * width; i += blockDim.x) {
-    const int r = i / width, c = i - r * width;
-    if (c >= r) tri[r * width - r * (r - 1) / 2 + c - r] = upper[(start + r) * columns + start + c];
-  }
-  __syncthreads();
-  if ((threadIdx.x & ~31) / kLanesPerRow >= rows_per_cta) return;       // whole warp without rows
-
-  const float inf = __int_as_float(0x7f800000);
-  for (int base = blockIdx.x * rows_per_cta; base < rows; base += gridDim.x * rows_per_cta) {
-    const int row = base + slot;
-    const bool active = slot < rows_per_cta && row < rows;
-    float* wr = w + static_cast<int64_t>(active ? row : 0) * columns + start;
-    for (int j = sl; j < width; j += kLanesPerRow) { open[j] = active ? wr[j] : 0.f; chosen[j] = 0; }
-    const float s = active ? scales[row] : 1.f;
-    float loss = active ? losses[row] : 0.f;
-    __syncwarp();
-    int off = 0;                                   // where row `index` of the triangle starts
-    for (int index = 0; index < width; ++index) {
-      if (index % group == 0) {
-        const int span = min(group, width - index);
-        const int remove = max(0, 2 - (group - span));
-        // the `remove` smallest scores of the group, ties to the lower column
-        float score = inf;
-        int g = 99;
-        if (sl < span) {
-          const int i = index + sl;
-          const float v = open[i], d = tri[i * width - i * (i - 1) / 2];
-          score = __fdiv_rn(__fmul_rn(v, v), __fmul_rn(d, d));
-          g = sl;
-        }
-        const int first = argmin8(score, g);
-        if (g == first) { score = inf; g = 99; }
-        const int second = argmin8(score, g);
-        if (sl == 0) {
-          if (remove > 0) chosen[index + first] = 1;
-          if (remove > 1) chosen[index + second] = 1;
-        }
-        __syncwarp();
-      }
-      const float current = open[index];
-      float fin = joint ? __fmul_rn(round_to_grid(current, s), s) : current;
-      if (chosen[index]) fin = 0.f;
-      const float e = __fdiv_rn(__fsub_rn(current, fin), tri[off]);
-      loss = __fadd_rn(loss, __fmul_rn(__fmul_rn(e, e), 0.5f));
-      __syncwarp();
-      if (sl == 0) { open[index] = fin; err[index] = e; }
-      const float* frow = tri + off - index;       // frow[j] = factor[index][j] for j >= index
-      if ((width & 3) == 0) {
-        // four columns per lane and step: one 16-byte read and write of the open values
-        float4* open4 = reinterpret_cast<float4*>(open);
-        for (int q4 = ((index + 1) >> 2) + sl; q4 < (width >> 2); q4 += kLanesPerRow) {
-          float4 o = open4[q4];
-          const int j = q4 << 2;
-          if (j > index) o.x = __fsub_rn(o.x, __fmul_rn(e, frow[j]));
-          if (j + 1 > index) o.y = __fsub_rn(o.y, __fmul_rn(e, frow[j + 1]));
-          if (j + 2 > index) o.z = __fsub_rn(o.z, __fmul_rn(e, frow[j + 2]));
-          o.w = __fsub_rn(o.w, __fmul_rn(e, frow[j + 3]));
-          open4[q4] = o;
-        }
-      } else {
-        for (int j = index + 1 + sl; j < width; j += kLanesPerRow) open[j] = __fsub_rn(open[j], __fmul_rn(e, frow[j]));
-      }
-      __syncwarp();
-      off += width - index;
+  for (int r = warp; r < width; r += warps) {
+    float* dst = tile + obs_row(r, width);
+    const float* src = upper + (start + r) * columns + start;
+    for (int c = (r & ~3) + lane; c < wp; c += 32) {
+      if (c < width) ptx::cp_async4(dst + c, src + c); else dst[c] = 0.f;
     }
-    if (active) {
-      uint8_t* zr = zeros + static_cast<int64_t>(row) * columns + start;
-      float* er = errors + static_cast<int64_t>(row) * width;
-      for (int j = sl; j < width; j += kLanesPerRow) { wr[j] = open[j]; er[j] = err[j]; zr[j] = chosen[j]; }
-      if (sl == 0) losses[row] = loss;
+  }
+  ptx::cp_async_wait_all();
+  __syncthreads();
+  bool in_range = true;
+  for (int i = threadIdx.x; i < width; i += blockDim.x) {
+    const float d = tile[obs_row(i, width) + i], dd = __fmul_rn(d, d);
+    recip[i] = __fdiv_rn(1.f, d);
+    square[i] = dd;
+    square_recip[i] = __fdiv_rn(1.f, dd);
+    in_range = in_range && within(d, 0x1p-15f, 0x1p15f);
+  }
+  const bool exact = __syncthreads_and(in_range);
+  const float inf = __int_as_float(0x7f800000);
+  float* open = open_all + slot * pitch;
+  float* err = err_all + slot * pitch;
+  uint8_t* chosen = chosen_all + slot * groups;
+
+  for (int base = blockIdx.x * rows_per_cta; base < rows; base += gridDim.x * rows_per_cta) {
+    const int row = base + slot, warp_row = base + warp * kRowsPerWarp;
+    // the warp's rows, one after the other, 128 bytes at a time, all in flight together
+    for (int r = 0; r < kRowsPerWarp; ++r) {
+      const float* wr = w + static_cast<int64_t>(warp_row + r) * columns + start;
+      float* to = open_all + (warp * kRowsPerWarp + r) * pitch;
+      for (int j = lane; j < wp; j += 32) {
+        if (warp_row + r < rows && j < width) ptx::cp_async4(to + j, wr + j); else to[j] = 0.f;
+      }
+    }
+    const float s = row < rows ? scales[row] : 1.f;
+    const float s_recip = __fdiv_rn(1.f, s);
+    const float v_limit = within(s, 0x1p-60f, 0x1p60f) ? 0x1p60f : -1.f;
+    float loss = row < rows ? losses[row] : 0.f;
+    ptx::cp_async_wait_all();
+    __syncwarp();
+    for (int group = 0; group < groups; ++group) {
+      const int i0 = group * G, span = min(G, width - i0);
+      float v[G], e[G];
+#pragma unroll
+      for (int c = 0; c < G; ++c) v[c] = c < span ? open[i0 + c] : 0.f;
+      // the two smallest scores (one or none in an incomplete group), ties to the lower column
+      const int remove = max(0, 2 - (G - span));
+      float low = inf, next = inf;
+      int first = G, second = G;
+#pragma unroll
+      for (int c = 0; c < G; ++c) {
+        if (c < span) {
+          const float vv = __fmul_rn(v[c], v[c]);
+          const float score = exact && (vv == 0.f || within(vv, 0x1p-90f, 0x1p60f)) ? quotient(vv, square[i0 + c], square_recip[i0 + c])
+                                                              : __fdiv_rn(vv, square[i0 + c]);
+          if (first == G || score < low) { next = low; second = first; low = score; first = c; }
+          else if (second == G || score < next) { next = score; second = c; }
+        }
+      }
+      const unsigned mask = (remove > 0 ? 1u << first : 0u) | (remove > 1 ? 1u << second : 0u);
+#pragma unroll
+      for (int c = 0; c < G; ++c) {
+        e[c] = 0.f;
+        if (c < span) {
+          const float* frow = tile + obs_row(i0 + c, width) + i0;      // frow[d] = factor[i0 + c][i0 + d]
+          float fin = v[c];
+          if (joint) {
+            float g;
+            if (fabsf(v[c]) <= v_limit) g = fminf(127.f, fmaxf(-128.f, copysignf(rintf(quotient(v[c], s, s_recip)), v[c])));
+            else g = round_to_grid(v[c], s);
+            fin = __fmul_rn(g, s);
+          }
+          if (mask >> c & 1u) fin = 0.f;
+          const float d = __fsub_rn(v[c], fin);
+          if (exact && within(d, 0x1p-90f, 0x1p60f)) e[c] = quotient(d, frow[c], recip[i0 + c]);
+          else e[c] = exact && d == 0.f ? __fmul_rn(d, recip[i0 + c]) : __fdiv_rn(d, frow[c]);
+          loss = __fadd_rn(loss, __fmul_rn(__fmul_rn(e[c], e[c]), 0.5f));
+          v[c] = fin;
+#pragma unroll
+          for (int o = c + 1; o < G; ++o) v[o] = __fsub_rn(v[o], __fmul_rn(e[c], frow[o]));
+        }
+      }
+      // The group's errors on the open columns: o = (o - e0 f0) - e1 f1 ..., two columns at a time.  The
+      // packed multiply and add of sm_100a are contracted to one rounding whatever their rounding
+      // modifiers say, so the product is made by a multiply-add onto a -0 that the compiler does not know
+      // (the same value, sign of zero included).
+      const float2 none = make_float2(minus_zero, minus_zero);
+      const int i1 = i0 + G;
+      if (i1 < width) {
+        const float* frow[G];
+        float2 minus[G];
+#pragma unroll
+        for (int c = 0; c < G; ++c) {
+          frow[c] = tile + obs_row(i0 + c, width);
+          minus[c] = make_float2(-e[c], -e[c]);
+        }
+        if (G == 6 && (i1 & 2) && sl == 0) {
+          float2 o = *reinterpret_cast<float2*>(open + i1);
+#pragma unroll
+          for (int c = 0; c < G; ++c)
+            o = __fadd2_rn(o, __ffma2_rn(minus[c], *reinterpret_cast<const float2*>(frow[c] + i1), none));
+          *reinterpret_cast<float2*>(open + i1) = o;
+        }
+        // two quads a step, so that one's chain hides the other's
+        for (int j = ((i1 + 3) & ~3) + 4 * sl; j < width; j += 8 * kLanesPerRow) {
+          const int jb = j + 4 * kLanesPerRow < width ? j + 4 * kLanesPerRow : j;
+          const float4 oa = *reinterpret_cast<const float4*>(open + j), ob = *reinterpret_cast<const float4*>(open + jb);
+          float2 o[4] = {make_float2(oa.x, oa.y), make_float2(oa.z, oa.w), make_float2(ob.x, ob.y), make_float2(ob.z, ob.w)};
+#pragma unroll
+          for (int c = 0; c < G; ++c) {
+            const float4 fa = *reinterpret_cast<const float4*>(frow[c] + j), fb = *reinterpret_cast<const float4*>(frow[c] + jb);
+            o[0] = __fadd2_rn(o[0], __ffma2_rn(minus[c], make_float2(fa.x, fa.y), none));
+            o[1] = __fadd2_rn(o[1], __ffma2_rn(minus[c], make_float2(fa.z, fa.w), none));
+            o[2] = __fadd2_rn(o[2], __ffma2_rn(minus[c], make_float2(fb.x, fb.y), none));
+            o[3] = __fadd2_rn(o[3], __ffma2_rn(minus[c], make_float2(fb.z, fb.w), none));
+          }
+          *reinterpret_cast<float4*>(open + jb) = make_float4(o[2].x, o[2].y, o[3].x, o[3].y);
+          *reinterpret_cast<float4*>(open + j) = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
+        }
+      }
+      __syncwarp();                   // every lane of the row has read the group's values
+#pragma unroll
+      for (int c = 0; c < G; ++c)
+        if (sl == (c & (kLanesPerRow - 1)) && c < span) { open[i0 + c] = v[c]; err[i0 + c] = e[c]; }
+      if (sl == 0) chosen[group] = static_cast<uint8_t>(mask);
+      __syncwarp();
+    }
+    if (sl == 0 && row < rows) losses[row] = loss;
+    for (int r = 0; r < kRowsPerWarp && warp_row + r < rows; ++r) {
+      const int at = warp * kRowsPerWarp + r;
+      const int64_t out = static_cast<int64_t>(warp_row + r) * columns + start;
+      float* er = errors + static_cast<int64_t>(warp_row + r) * width;
+      for (int j = lane; j < width; j += 32) {
+        w[out + j] = open_all[at * pitch + j];
+        er[j] = err_all[at * pitch + j];
+        zeros[out + j] = chosen_all[at * groups + j / G] >> (j % G) & 1u;
+      }
     }
     __syncwarp();
   }
 }
 
 // w[r, stop + j] -= sum_k errors[r, k] * upper[start + k, stop + j], the sum taken as
-// acc = fma(e, u, acc) from acc = 0 in increasing k.  128 x 128 output tile, 8 x 8 per thread
-// (rows ty*4+i and 64+ty*4+i, columns likewise, so shared-memory reads are conflict-free float4s),
-// the next k-slab fetched into registers while the current one is multiplied.
+// acc = fma(e, u, acc) from acc = 0 in increasing k.  Bound by the FP32 pipes and, next to them, the
+// shared-memory port: 128 x 128 output tile, 8 x 16 per thread (rows ty*4+i and 64+ty*4+i, columns
+// 32*h+tx*4+j) in the packed form of two multiply-adds, so that six 16-byte reads feed 64 of them.  Two
+// slabs: the next one's B comes in by asynchronous copies, its A through registers, while the current one
+// is multiplied.  VEC: 16-byte accesses of the factor, the errors and w (all rows 16-byte aligned).
+// 8 x 8 per thread, scalar multiply-adds, scalar loads, one slab: 202 us a block (26 TFLOP/s) at 9216 x
+// 3072 in blocks of 192; packed multiply-adds and two slabs alone 174 us; this form 148 us.
 constexpr int kTileM = 128, kTileN = 128, kTileK = 16;
 
-__global__ void __launch_bounds__(256)
+template <bool VEC>
+__global__ void __launch_bounds__(128, 2)
 obs_trailing_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start, int width,
                     const float* __restrict__ upper, const float* __restrict__ errors) {
-  __shared__ __align__(16) float a_s[kTileK][kTileM];
-  __shared__ __align__(16) float b_s[kTileK][kTileN];
+  __shared__ __align__(16) float a_s[2][kTileK][kTileM];
+  __shared__ __align__(16) float b_s[2][kTileK][kTileN];
   const int64_t stop = start + width;
   const int cols = static_cast<int>(columns - stop);
   const int row0 = blockIdx.y * kTileM, col0 = blockIdx.x * kTileN;
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  // this thread's share of a slab: 8 consecutive k of one row of A, 8 consecutive columns of one k of B
-  const int a_row = t >> 1, a_k = (t & 1) * 8;
-  const int b_k = t >> 4, b_col = (t & 15) * 8;
-  const float* a_src = errors + static_cast<int64_t>(row0 + a_row) * width;
-  const bool a_ok = row0 + a_row < rows;
-  float a_reg[8], b_reg[8];
-  auto fetch = [&](int k0) {
+  const int t = threadIdx.x, tx = t & 7, ty = t >> 3;
+  // this thread's share of a slab: the 16 k of one row of A, 16 columns of one k of B
+  const float* a_src = errors + static_cast<int64_t>(row0 + t) * width;
+  const bool a_ok = row0 + t < rows;
+  float a_reg[kTileK];
+  auto fetch_a = [&](int k0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) a_reg[i] = (a_ok && k0 + a_k + i < width) ? a_src[k0 + a_k + i] : 0.f;
-    const bool k_ok = k0 + b_k < width;
-    const float* b_src = upper + (start + k0 + b_k) * columns + stop + col0 + b_col;
+    for (int i = 0; i < kTileK; i += 4) {
+      if constexpr (VEC) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a_ok && k0 + i < width) v = *reinterpret_cast<const float4*>(a_src + k0 + i);
+        a_reg[i] = v.x; a_reg[i + 1] = v.y; a_reg[i + 2] = v.z; a_reg[i + 3] = v.w;
+      } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) b_reg[i] = (k_ok && col0 + b_col + i < cols) ? b_src[i] : 0.f;
+        for (int j = i; j < i + 4; ++j) a_reg[j] = a_ok && k0 + j < width ? a_src[k0 + j] : 0.f;
+      }
+    }
   };
-  float acc[8][8] = {};
-  fetch(0);
-  for (int k0 = 0; k0 < width; k0 += kTileK) {
+  auto store_a = [&](int slab) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { a_s[a_k + i][a_row] = a_reg[i]; b_s[b_k][b_col + i] = b_reg[i]; }
-    __syncthreads();
-    if (k0 + kTileK < width) fetch(k0 + kTileK);
+    for (int i = 0; i < kTileK; ++i) a_s[slab][i][t] = a_reg[i];
+  };
+  auto fetch_b = [&](int k0, int slab) {
+    const bool k_ok = k0 + ty < width;
+    const float* src = upper + (start + (k_ok ? k0 + ty : 0)) * columns + stop;
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+      for (int j = 0; j < 4; j += VEC ? 4 : 1) {
+        const int c = 32 * h + tx * 4 + j;
+        const bool in = k_ok && col0 + c < cols;                   // VEC: cols is a multiple of four
+        const float* from = src + (in ? col0 + c : 0);
+        if constexpr (VEC) ptx::cp_async16(&b_s[slab][ty][c], from, in ? 16u : 0u);
+        else ptx::cp_async4(&b_s[slab][ty][c], from, in ? 4u : 0u);
+      }
+  };
+  float2 acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  fetch_a(0);
+  fetch_b(0, 0);
+  store_a(0);
+  ptx::cp_async_wait_all();
+  __syncthreads();
+  int slab = 0;
+  for (int k0 = 0; k0 < width; k0 += kTileK, slab ^= 1) {
+    const bool more = k0 + kTileK < width;
+    if (more) { fetch_b(k0 + kTileK, slab ^ 1); fetch_a(k0 + kTileK); }
 #pragma unroll
     for (int k = 0; k < kTileK; ++k) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&a_s[k][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&a_s[k][64 + ty * 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&b_s[k][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&b_s[k][64 + tx * 4]);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      float2 b[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int h = 0; h < 4; ++h) {
+        const float4 v = *reinterpret_cast<const float4*>(&b_s[slab][k][32 * h + tx * 4]);
+        b[2 * h] = make_float2(v.x, v.y);
+        b[2 * h + 1] = make_float2(v.z, v.w);
+      }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = __fmaf_rn(a[i], b[j], acc[i][j]);
+      for (int h = 0; h < 2; ++h) {
+        const float4 v = *reinterpret_cast<const float4*>(&a_s[slab][k][64 * h + ty * 4]);
+        const float a[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[4 * h + i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[4 * h + i][j]);
+      }
     }
-    __syncthreads();
+    if (more) {
+      store_a(slab ^ 1);
+      ptx::cp_async_wait_all();
+      __syncthreads();
+    }
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int r = row0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
     if (r >= rows) continue;
+    float* wr = w + static_cast<int64_t>(r) * columns + stop;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int c = col0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-      if (c >= cols) continue;
-      float* p = w + static_cast<int64_t>(r) * columns + stop + c;
-      *p = __fsub_rn(*p, acc[i][j]);
+    for (int h = 0; h < 4; ++h) {
+      const int c = col0 + 32 * h + tx * 4;
+      const float2 lo = acc[i][2 * h], hi = acc[i][2 * h + 1];
+      if constexpr (VEC) {
+        if (c < cols) {
+          float4 v = *reinterpret_cast<float4*>(wr + c);
+          v = make_float4(__fsub_rn(v.x, lo.x), __fsub_rn(v.y, lo.y), __fsub_rn(v.z, hi.x), __fsub_rn(v.w, hi.y));
+          *reinterpret_cast<float4*>(wr + c) = v;
+        }
+      } else {
+        const float sum[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (c + j < cols) wr[c + j] = __fsub_rn(wr[c + j], sum[j]);
+      }
     }
   }
 }
 
 // Final export: q = clamp(rint(w / scale)) with the selected zeros forced to 0; status bit 0 is set
 // when q * scale differs from w (checked only when check_grid), bit 1 when a complete group holds
-// more than group - 2 nonzeros.  One thread per (row, group).
-__global__ void obs_finish_kernel(const float* __restrict__ w, const float* __restrict__ scales,
-                                  const uint8_t* __restrict__ zeros, int rows, int64_t columns, int group,
-                                  int check_grid, int8_t* __restrict__ q, int32_t* __restrict__ status) {
-  const int64_t groups = (columns + group - 1) / group;
-  const int64_t id = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (id >= rows * groups) return;
-  const int64_t row = id / groups, g = id - row * groups;
+// more than group - 2 nonzeros, bit 2 when w holds a non-finite value.  Bound by HBM: a CTA per row, a
+// thread per group, two columns at a time where the rows allow it (PAIRS).  One thread per group over the
+// whole weight, its row found by a 64-bit division: 91 us at 9216 x 3072 (4:6); now 43 us.
+template <int G, bool PAIRS>
+__global__ void __launch_bounds__(256)
+obs_finish_kernel(const float* __restrict__ w, const float* __restrict__ scales, const uint8_t* __restrict__ zeros,
+                  int64_t columns, int check_grid, int8_t* __restrict__ q, int32_t* __restrict__ status) {
+  const int64_t row = blockIdx.x;
   const float s = scales[row];
-  int nonzero = 0, flags = 0;
-  const int64_t base = row * columns;
-  for (int64_t c = g * group; c < min(columns, (g + 1) * group); ++c) {
-    const float v = w[base + c];
-    int value = static_cast<int>(round_to_grid(v, s));
-    if (zeros[base + c]) value = 0;
-    q[base + c] = static_cast<int8_t>(value);
-    nonzero += value != 0;
-    if (check_grid && !(__fmul_rn(static_cast<float>(value), s) == v)) flags |= 1;
+  w += row * columns;
+  zeros += row * columns;
+  q += row * columns;
+  int flags = 0;
+  for (int64_t c0 = static_cast<int64_t>(threadIdx.x) * G; c0 < columns; c0 += static_cast<int64_t>(blockDim.x) * G) {
+    const int span = static_cast<int>(columns - c0 < G ? columns - c0 : G);
+    int nonzero = 0;
+    auto column = [&](float v, bool zero) {
+      const int value = zero ? 0 : static_cast<int>(round_to_grid(v, s));
+      nonzero += value != 0;
+      if (check_grid && !(__fmul_rn(static_cast<float>(value), s) == v)) flags |= 1;
+      if (!isfinite(v)) flags |= 4;
+      return static_cast<char>(value);
+    };
+#pragma unroll
+    for (int c = 0; c < G; c += PAIRS ? 2 : 1) {
+      if (c < span) {
+        if constexpr (PAIRS) {
+          const float2 v = *reinterpret_cast<const float2*>(w + c0 + c);
+          const uchar2 z = *reinterpret_cast<const uchar2*>(zeros + c0 + c);
+          *reinterpret_cast<char2*>(q + c0 + c) = make_char2(column(v.x, z.x), column(v.y, z.y));
+        } else {
+          q[c0 + c] = column(w[c0 + c], zeros[c0 + c]);
+        }
+      }
+    }
+    if (span == G && nonzero > G - 2) flags |= 2;
   }
-  if ((g + 1) * group <= columns && nonzero > group - 2) flags |= 2;
   if (flags) atomicOr(status, flags);
 }
 
@@ -223,16 +384,13 @@ __global__ void obs_finish_kernel(const float* __restrict__ w, const float* __re
 
 using namespace ss;
 
-static size_t obs_block_smem(int64_t width) {
-  const int64_t triangle = (width * (width + 1) / 2 + 3) / 4 * 4;
-  return static_cast<size_t>(triangle + kRowsPerCta * 2 * width) * sizeof(float) + kRowsPerCta * width;
+static size_t obs_block_smem(int width, int group, int rows) {
+  const int wp = (width + 3) & ~3;
+  return (static_cast<size_t>(obs_tile_floats(width)) + 3 * wp + 2 * rows * obs_pitch(width)) * sizeof(float) +
+         static_cast<size_t>(rows) * ((width + group - 1) / group);
 }
 
-extern "C" int ss_obs_max_blocksize(void) {
-  int64_t width = 8;
-  while (obs_block_smem(width + 1) <= 227 * 1024) ++width;
-  return static_cast<int>(width);
-}
+extern "C" int ss_obs_max_blocksize(void) { return kObsMaxWidth; }
 
 extern "C" int ss_obs_block(float* w, int64_t rows, int64_t columns, int64_t start, int64_t width,
                             const float* upper, const float* scales, int group, int joint,
@@ -242,21 +400,24 @@ extern "C" int ss_obs_block(float* w, int64_t rows, int64_t columns, int64_t sta
   SS_REQUIRE(rows > 0 && rows < (1ll << 31) && columns > 0 && columns < (1ll << 31), SS_E_ARG, "obs_block: invalid shape");
   SS_REQUIRE(start >= 0 && width > 0 && start + width <= columns && start % group == 0, SS_E_ARG,
              "obs_block: the block [start, start+width) must lie inside the row and start on a group boundary");
-  const size_t smem = obs_block_smem(width);
-  SS_REQUIRE(smem <= 227 * 1024, SS_E_ARG, "obs_block: a block of %lld columns needs %zu bytes of shared memory (limit 232448)",
-             static_cast<long long>(width), smem);
-  SS_CUDA(cudaFuncSetAttribute(obs_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  SS_REQUIRE(width <= kObsMaxWidth, SS_E_ARG, "obs_block: a block of %lld columns does not fit shared memory (limit %d)",
+             static_cast<long long>(width), kObsMaxWidth);
   int device = 0, sms = 0;
   SS_CUDA(cudaGetDevice(&device));
   SS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  // spread the rows over all SMs: a CTA takes up to kRowsPerCta rows per pass, whole warps of 4
-  int64_t per_cta = ((rows + sms - 1) / sms + 3) / 4 * 4;
-  if (per_cta > kRowsPerCta) per_cta = kRowsPerCta;
+  // spread the rows over all SMs, whole warps of eight; the widest blocks leave room for 56 rows
+  int64_t per_cta = ((rows + sms - 1) / sms + kRowsPerWarp - 1) / kRowsPerWarp * kRowsPerWarp;
+  if (per_cta > kObsMaxRows) per_cta = kObsMaxRows;
+  const int wide = static_cast<int>(width);
+  while (obs_block_smem(wide, group, static_cast<int>(per_cta)) > 227 * 1024) per_cta -= kRowsPerWarp;
+  const size_t smem = obs_block_smem(wide, group, static_cast<int>(per_cta));
   const int64_t wanted = (rows + per_cta - 1) / per_cta;
   const unsigned grid = static_cast<unsigned>(wanted < sms ? wanted : sms);
-  obs_block_kernel<<<grid, kObsWarps * 32, smem, static_cast<cudaStream_t>(stream)>>>(
-      w, static_cast<int>(rows), columns, start, static_cast<int>(width), static_cast<int>(per_cta), upper, scales,
-      group, joint != 0, zeros, errors, losses);
+  auto kernel = group == 4 ? obs_block_kernel<4> : group == 6 ? obs_block_kernel<6> : obs_block_kernel<8>;
+  SS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  kernel<<<grid, static_cast<unsigned>(per_cta) * kLanesPerRow, smem, static_cast<cudaStream_t>(stream)>>>(
+      w, static_cast<int>(rows), columns, start, wide, static_cast<int>(per_cta), upper, scales, joint != 0, -0.0f, zeros,
+      errors, losses);
   SS_CUDA(cudaGetLastError());
   return SS_OK;
 }
@@ -270,7 +431,10 @@ extern "C" int ss_obs_trailing(float* w, int64_t rows, int64_t columns, int64_t 
   if (cols == 0) return SS_OK;
   const dim3 grid(static_cast<unsigned>((cols + kTileN - 1) / kTileN), static_cast<unsigned>((rows + kTileM - 1) / kTileM));
   SS_REQUIRE(grid.y <= 65535, SS_E_ARG, "obs_trailing: too many rows for one launch");
-  obs_trailing_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  const bool vec = ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(upper) | reinterpret_cast<uintptr_t>(errors)) & 15) == 0 &&
+                   columns % 4 == 0 && width % 4 == 0 && start % 4 == 0;
+  auto kernel = vec ? obs_trailing_kernel<true> : obs_trailing_kernel<false>;
+  kernel<<<grid, 128, 0, static_cast<cudaStream_t>(stream)>>>(
       w, static_cast<int>(rows), columns, start, static_cast<int>(width), upper, errors);
   SS_CUDA(cudaGetLastError());
   return SS_OK;
@@ -282,10 +446,15 @@ extern "C" int ss_obs_finish(const float* w, const float* scales, const uint8_t*
   SS_REQUIRE(w && scales && zeros && qweight && status, SS_E_ARG, "obs_finish: null pointer");
   SS_REQUIRE(mode_ok(group), SS_E_ARG, "obs_finish: group must be 4, 6 or 8");
   SS_REQUIRE(rows > 0 && rows < (1ll << 31) && columns > 0 && columns < (1ll << 31), SS_E_ARG, "obs_finish: invalid shape");
-  const int64_t total = rows * ((columns + group - 1) / group);
-  SS_REQUIRE((total + 255) / 256 < (1ll << 31), SS_E_ARG, "obs_finish: weight too large for one launch");
-  obs_finish_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      w, scales, zeros, static_cast<int>(rows), columns, group, check_grid, qweight, status);
+  const bool pairs = columns % 2 == 0 && (reinterpret_cast<uintptr_t>(w) & 7) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(zeros) | reinterpret_cast<uintptr_t>(qweight)) & 1) == 0;
+  auto kernel = group == 4 ? (pairs ? obs_finish_kernel<4, true> : obs_finish_kernel<4, false>)
+              : group == 6 ? (pairs ? obs_finish_kernel<6, true> : obs_finish_kernel<6, false>)
+                           : (pairs ? obs_finish_kernel<8, true> : obs_finish_kernel<8, false>);
+  const int64_t groups = (columns + group - 1) / group;
+  const unsigned threads = groups >= 256 ? 256u : static_cast<unsigned>((groups + 31) / 32 * 32);
+  kernel<<<static_cast<unsigned>(rows), threads, 0, static_cast<cudaStream_t>(stream)>>>(w, scales, zeros, columns, check_grid,
+                                                                                       qweight, status);
   SS_CUDA(cudaGetLastError());
   return SS_OK;
 }

@@ -162,3 +162,30 @@ def test_full_size_weight_sample_rows_equal_the_oracle(recon, oracle_c):
     assert np.array_equal(result["zeros"][pick].cpu().numpy(), expect_zeros)
     assert np.array_equal(_bits(result["compensated"][pick]), expect_w.view(np.uint32))
     assert np.array_equal(_bits(result["proxy_loss"][pick]), expect_loss.view(np.uint32))
+
+
+@pytest.mark.parametrize("rows,columns,group,blocksize,method,weight_factor,input_factor", [
+    (70, 411, 6, 54, "joint", 1.0, 1.0),           # rows of the factor and of w off 16 bytes, odd tail
+    (9600, 20, 4, 8, "joint", 1.0, 1.0),           # more rows than one pass of all CTAs holds
+    (9, 225, 8, 224, "prune_then_rtn", 1.0, 1.0),  # a block of one column behind the widest one
+    (40, 96, 8, 48, "joint", 1.0, 2.0 ** 17),      # divisors below the range of the reciprocal form
+    (40, 96, 6, 48, "joint", 2.0 ** -64, 1.0),     # scales below it, dividends among them
+    (40, 96, 4, 48, "joint", 2.0 ** 64, 1.0),      # and above
+])
+def test_kernels_match_the_oracle_at_the_edges(recon, oracle_c, rows, columns, group, blocksize, method, weight_factor,
+                                               input_factor):
+    weight, hessian = _synthetic(rows, columns, seed=rows + columns)
+    weight, hessian = weight * weight_factor, hessian * input_factor ** 2
+    weight[::3, ::5] = 0
+    curvature = recon.factor_hessian(hessian)
+    scales = recon.channel_scales(weight)
+    q, zeros, w, losses = oracle_c.obs_compress(weight.numpy(), curvature.upper.numpy(), curvature.dead.numpy(),
+                                                scales.numpy(), group, blocksize, method == "joint")
+    dev = "cuda:0"
+    on_gpu = recon.Curvature(curvature.upper.to(dev), curvature.dead.to(dev), curvature.damping)
+    result = recon.compress(weight.to(dev), on_gpu, group, method=method, blocksize=blocksize,
+                            allow_tail=bool(columns % group))
+    assert np.array_equal(result["zeros"].cpu().numpy(), zeros)
+    assert np.array_equal(result["qweight"].cpu().numpy(), q)
+    assert np.array_equal(_bits(result["compensated"]), w.view(np.uint32))
+    assert np.array_equal(_bits(result["proxy_loss"]), losses.view(np.uint32))
