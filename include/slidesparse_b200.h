@@ -167,6 +167,11 @@ int ss_quantize_lift_fused(const void* x_bf16, int64_t x_row_stride, int64_t m, 
                            int prologue, const void* shift_bf16, const void* scale_bf16,
                            int64_t mod_row_stride, int64_t rows_per_batch, float eps,
                            int8_t* q, float* sa, void* stream);
+/* out[r, c] = bf16(x[r, c] + gate[r / rows_per_batch, c] * y[r, c]), BF16, one rounding: the gated residual
+ * behind an attention output projection.  x, y and out are dense [rows, n], gate rows lie gate_row_stride
+ * elements apart; all 16-byte aligned, n and the stride multiples of 8.  No counterpart in the reference. */
+int ss_gate_add(const void* x_bf16, const void* gate_bf16, int64_t gate_row_stride, const void* y_bf16, void* out_bf16,
+                int64_t rows, int64_t rows_per_batch, int64_t n, void* stream);
 /* ss_quantize_lift_fused followed by the GEMM.  No counterpart in the reference (see above);
  * the remaining arguments are those of ss_projection, plus an optional gated accumulation, the
  * other element-wise neighbour of an FFN-out projection: with gate_bf16 != NULL (BF16

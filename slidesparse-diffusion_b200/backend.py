@@ -151,6 +151,7 @@ def _declare(lib):
         "ss_quantize_lift_fused": [vp, i64, i64, i64, i32, i32, vp, vp, i64, i64, c.c_float, vp, vp, vp],
         "ss_projection_fused": [vp, i64, i64, i64, i32, i32, vp, vp, i64, i64, c.c_float,
                                 vp, vp, vp, vp, vp, i64, vp, i64, i64, i64, vp, vp, vp, i64, vp],
+        "ss_gate_add": [vp, vp, i64, vp, vp, i64, i64, i64, vp],
         "ss_projection_peers": [vp, i64, i64, i64, i32, vp, vp, vp, vp, i64, i64, vp, vp, vp, i32, i64, vp],
         "ss_projection_static": [vp, i64, i64, i64, i32, vp, vp, vp, vp, i64, i64, vp, i64, vp],
         "ss_plan_create": [vp, vp, vp, vp, i64, i64, i64, i64, i32, vp],
@@ -541,6 +542,16 @@ def quantize_lift_fused(input, group, prologue):
     return q, sa
 
 
+def gate_add(x, gate, y):
+    """x + gate[:, None] * y with BF16 x, y [batch, rows, n] and gate [batch, n]: one kernel where the
+    library is loaded and nothing has to be differentiated or traced, torch.addcmul otherwise."""
+    if (_ops_registered and x.is_cuda and x.dtype == y.dtype == gate.dtype == torch.bfloat16
+            and not (torch.is_grad_enabled() and (x.requires_grad or y.requires_grad or gate.requires_grad))
+            and not torch.compiler.is_compiling()):
+        return torch.ops.slidesparse_b200.gate_add(x, gate, y)
+    return torch.addcmul(x, gate[:, None], y)
+
+
 def projection_fused(input, prologue, packed, metadata, scales, bias, group, n, output_addend=None,
                      gate=None, residual=None):
     """`projection` with the prologue applied to the input inside the front-end kernel.
@@ -773,6 +784,8 @@ def _register_ops(binding):
     own.define(f"projection_fused(Tensor input,{pro},{weights},Tensor? output_addend=None)->Tensor")
     own.define(f"projection_fused_accumulate_(Tensor(a!) residual,Tensor input,{pro},{weights},Tensor gate)->()")
 
+    own.define("gate_add(Tensor x,Tensor gate,Tensor y)->Tensor")
+
     def _prologue_of(code, shift, scale, eps):
         kind = {v: k for k, v in PROLOGUES.items()}[int(code)]
         return Prologue(kind, shift, scale, eps)
@@ -796,6 +809,7 @@ def _register_ops(binding):
         for name in ("projection", "projection_packed16", "projection_scalar"):
             mild.impl(name, _projection, "CUDA")
         prepared.impl("run", _prepared_run, "CUDA")
+        own.impl("gate_add", lambda x, gate, y: torch.addcmul(x, gate[:, None], y), "CUDA")
         own.impl("projection_fused", _op_fused, "CUDA")
         own.impl("projection_fused_accumulate_", _op_fused_accumulate, "CUDA")
     _libraries.append(own)
@@ -803,6 +817,10 @@ def _register_ops(binding):
     @torch.library.register_fake("slidesparse_b200::projection_fused")
     def _fake_fused(input, prologue, shift, scale, eps, packed, metadata, scales, bias, group, n, output_addend=None):
         return input.new_empty((*input.shape[:-1], n))
+
+    @torch.library.register_fake("slidesparse_b200::gate_add")
+    def _fake_gate_add(x, gate, y):
+        return torch.empty_like(x)
 
     @torch.library.register_fake("slidesparse_b200::projection_fused_accumulate_")
     def _fake_fused_accumulate(residual, input, prologue, shift, scale, eps, packed, metadata, scales, bias, group, n, gate):

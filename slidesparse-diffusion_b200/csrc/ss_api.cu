@@ -152,6 +152,11 @@ extern "C" int ss_quantize_lift_fused(const void* x, int64_t sx, int64_t m, int6
                                     eps, q, sa, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int ss_gate_add(const void* x, const void* gate, int64_t gate_stride, const void* y, void* out, int64_t rows,
+                           int64_t rows_per_batch, int64_t n, void* stream) {
+  return launch_gate_add(x, gate, gate_stride, y, out, rows, rows_per_batch, n, static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int ss_projection_fused(const void* x, int64_t sx, int64_t m, int64_t k, int group,
                                    int prologue, const void* shift, const void* scale,
                                    int64_t mod_stride, int64_t rows_per_batch, float eps,

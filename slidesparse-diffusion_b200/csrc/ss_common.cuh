@@ -76,6 +76,9 @@ int launch_quantize_lift_fused(const void* x, int64_t sx, int64_t m, int64_t k, 
                                const void* shift, const void* scale, int64_t mod_stride,
                                int64_t rows_per_batch, float eps, int8_t* q, float* sa, cudaStream_t stream);
 
+int launch_gate_add(const void* x, const void* gate, int64_t gate_stride, const void* y, void* out, int64_t rows,
+                    int64_t rows_per_batch, int64_t n, cudaStream_t stream);
+
 struct GemmArgs {
   const int8_t* q;
   const int8_t* packed;

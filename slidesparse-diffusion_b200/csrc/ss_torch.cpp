@@ -294,6 +294,23 @@ void projection_fused_accumulate(const Tensor& residual, const Tensor& input, in
   projection_fused_into(input, prologue, shift, scale, eps, packed, metadata, scales, bias, group, n, std::nullopt, &gate, out);
 }
 
+// x + gate[:, None] * y: one pass of this library's kernel where the rows allow it, torch's otherwise
+Tensor gate_add(const Tensor& x, const Tensor& gate, const Tensor& y) {
+  auto aligned = [](const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
+  const bool usable = x.dim() == 3 && x.numel() > 0 && y.sizes() == x.sizes() && gate.dim() == 2 && gate.size(0) == x.size(0) &&
+                      gate.size(1) == x.size(2) && x.scalar_type() == at::kBFloat16 && y.scalar_type() == at::kBFloat16 &&
+                      gate.scalar_type() == at::kBFloat16 && x.is_cuda() && y.device() == x.device() && gate.device() == x.device() &&
+                      x.is_contiguous() && y.is_contiguous() && x.size(2) % 8 == 0 && gate.stride(1) == 1 &&
+                      (gate.size(0) == 1 || (gate.stride(0) % 8 == 0 && gate.stride(0) >= gate.size(1))) &&
+                      aligned(x) && aligned(y) && aligned(gate) && x.size(0) * x.size(1) < (1ll << 31) && x.size(2) < (1ll << 31);
+  if (!usable) return at::addcmul(x, gate.unsqueeze(1), y);
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = new_output(x, x.size(2));
+  check(ss_gate_add(x.data_ptr(), gate.data_ptr(), gate.size(0) > 1 ? gate.stride(0) : gate.size(1), y.data_ptr(), out.data_ptr(),
+                    x.size(0) * x.size(1), x.size(1), x.size(2), current_stream(x)));
+  return out;
+}
+
 }  // namespace
 
 TORCH_LIBRARY_IMPL(sdacc_dualscale_sm80, CUDA, m) { m.impl("run", TORCH_FN(gemm_run)); }
@@ -313,4 +330,5 @@ TORCH_LIBRARY_IMPL(sdacc_prepared_projection_sm80, CUDA, m) { m.impl("run", TORC
 TORCH_LIBRARY_IMPL(slidesparse_b200, CUDA, m) {
   m.impl("projection_fused", TORCH_FN(projection_fused));
   m.impl("projection_fused_accumulate_", TORCH_FN(projection_fused_accumulate));
+  m.impl("gate_add", TORCH_FN(gate_add));
 }

@@ -16,7 +16,7 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
-from .backend import Prologue
+from .backend import Prologue, gate_add
 from .routing import ProjectionState, OrdinaryProxy, pack_members
 
 
@@ -87,7 +87,7 @@ def grid_embedding(grid, dim):
 
 def gate(x, g, y):
     """x + g[b] * y with g BF16 [batch, hidden]."""
-    return torch.addcmul(x, g[:, None], y)
+    return gate_add(x, g, y)
 
 
 def norm_modulate(shift, scale):
@@ -173,8 +173,9 @@ class DiTBlock(nn.Module):
         self.attn, self.ff = RoutedAttention(h, spec.heads), RoutedFeedForward(h, spec.mlp)
         self.adaln = nn.Linear(h, 6 * h)
 
-    def forward(self, x, c, context=None):
-        s1, c1, g1, s2, c2, g2 = self.adaln(F.silu(c)).chunk(6, dim=-1)
+    def forward(self, x, c, context=None, act=None):
+        """act: silu(c), where the caller has it (it is the same for every block)."""
+        s1, c1, g1, s2, c2, g2 = self.adaln(F.silu(c) if act is None else act).chunk(6, dim=-1)
         x = gate(x, g1, self.attn(x, prologue=norm_modulate(s1, c1)))
         return self.ff(x, norm_modulate(s2, c2), gated_residual=(x, g2))
 
@@ -211,8 +212,8 @@ class JointBlock(nn.Module):
         self.adaln = nn.Linear(h, 6 * h)
         self.adaln_text = nn.Linear(h, (2 if last else 6) * h)
 
-    def forward(self, x, text, c):
-        act = F.silu(c)
+    def forward(self, x, text, c, act=None):
+        act = F.silu(c) if act is None else act
         s1, c1, g1, s2, c2, g2 = self.adaln(act).chunk(6, dim=-1)
         mod_text = self.adaln_text(act).chunk(2 if self.last else 6, dim=-1)
         q, k, v = self.attn.qkv(x, prologue=norm_modulate(s1, c1))
@@ -336,19 +337,22 @@ class Denoiser(nn.Module):
         x = self.embed(self.patchify(latent)) + self.pos.to(latent.dtype)
         if spec.family == "dit":
             c = self.time(t) + self.classes(cond)
+            act = F.silu(c)
             for block in self.blocks:
-                x = block(x, c)
+                x = block(x, c, act=act)
         elif spec.family == "pixart":
             c = self.time(t)
-            c6, context = self.adaln_single(F.silu(c)), self.caption(cond)
+            act = F.silu(c)
+            c6, context = self.adaln_single(act), self.caption(cond)
             for block in self.blocks:
                 x = block(x, c6, context)
         else:
             text, pooled = cond
             c, text = self.time(t, pooled), self.context(text)
+            act = F.silu(c)
             for block in self.blocks:
-                x, text = block(x, text, c)
-        shift, scale = self.final_adaln(F.silu(c)).chunk(2, dim=-1)
+                x, text = block(x, text, c, act)
+        shift, scale = self.final_adaln(act).chunk(2, dim=-1)
         return self.unpatchify(self.final(norm_modulate(shift, scale).torch_reference(x)))
 
 
