@@ -36,8 +36,79 @@ __device__ __forceinline__ float round_to_grid(float v, float s) {
 }
 
 // Ranges in which quotient() is exact: divisors 2^-15 .. 2^15 (their squares 2^-30 .. 2^30), scales
-// 2^-60 .. 2^60, dividends 2^-90 .. 2^60.  Outside (and for NaN) the IEEE division runs.
+// 2^-60 .. 2^60, dividends +0 and 2^-90 .. 2^60.  Outside (and for NaN) the IEEE division runs.
 __device__ __forceinline__ bool within(float v, float lo, float hi) { return fabsf(v) >= lo && fabsf(v) <= hi; }
+__device__ __forceinline__ bool dividend_ok(float v) {
+  const uint32_t bits = __float_as_uint(v), lo = (127u - 90u) << 23, hi = (127u + 60u) << 23;
+  return bits == 0u || (bits & 0x7fffffffu) - lo <= hi - lo;
+}
+
+// The columns of one group while it is walked: values (which become the finalised ones) and errors.
+template <int G>
+struct ObsGroup {
+  float v[G], e[G], loss;
+  unsigned mask;
+};
+
+// Walks a group: the two smallest scores (one or none in an incomplete group, ties to the lower column)
+// are selected, then column by column it is rounded, its error taken and the group's later columns
+// updated.  FAST divides by the reciprocals and returns whether every division was within their range.
+template <int G, bool FAST>
+__device__ __forceinline__ bool walk_group(ObsGroup<G>& g, int i0, int span, const float* const (&row)[G], const float* recip,
+                                           const float* square, const float* square_recip, float s, float s_recip,
+                                           float v_limit, int joint) {
+  bool ok = true;
+  const int remove = max(0, 2 - (G - span));
+  float low = 0.f, next = 0.f;
+  int first = G, second = G;
+#pragma unroll
+  for (int c = 0; c < G; ++c) {
+    if (c < span) {
+      const float vv = __fmul_rn(g.v[c], g.v[c]);
+      float score;
+      if constexpr (FAST) {
+        score = quotient(vv, square[c], square_recip[c]);
+        ok = ok && dividend_ok(vv);
+      } else {
+        score = __fdiv_rn(vv, square[c]);
+      }
+      if (first == G || score < low) { next = low; second = first; low = score; first = c; }
+      else if (second == G || score < next) { next = score; second = c; }
+    }
+  }
+  g.mask = (remove > 0 ? 1u << first : 0u) | (remove > 1 ? 1u << second : 0u);
+#pragma unroll
+  for (int c = 0; c < G; ++c) {
+    g.e[c] = 0.f;
+    if (c < span) {
+      const float* frow = row[c] + i0;                 // frow[o] = factor[i0 + c][i0 + o]
+      float fin = g.v[c];
+      if (joint) {
+        float q;
+        if constexpr (FAST) {
+          q = fminf(127.f, fmaxf(-128.f, copysignf(rintf(quotient(g.v[c], s, s_recip)), g.v[c])));
+          ok = ok && fabsf(g.v[c]) <= v_limit;
+        } else {
+          q = round_to_grid(g.v[c], s);
+        }
+        fin = __fmul_rn(q, s);
+      }
+      if (g.mask >> c & 1u) fin = 0.f;
+      const float d = __fsub_rn(g.v[c], fin);
+      if constexpr (FAST) {
+        g.e[c] = quotient(d, frow[c], recip[c]);
+        ok = ok && dividend_ok(d);
+      } else {
+        g.e[c] = __fdiv_rn(d, frow[c]);
+      }
+      g.loss = __fadd_rn(g.loss, __fmul_rn(__fmul_rn(g.e[c], g.e[c]), 0.5f));
+      g.v[c] = fin;
+#pragma unroll
+      for (int o = c + 1; o < G; ++o) g.v[o] = __fsub_rn(g.v[o], __fmul_rn(g.e[c], frow[o]));
+    }
+  }
+  return ok;
+}
 
 __host__ __device__ __forceinline__ int obs_pitch(int width) {
   // floats between two rows' open values: 16 (mod 32), so that the 16-byte accesses of two rows'
@@ -52,12 +123,23 @@ __host__ __device__ __forceinline__ int obs_row(int i, int width) {
 }
 __host__ __device__ __forceinline__ int obs_tile_floats(int width) { return obs_row(width, width) + (width & ~3); }
 
+// The same with IEEE divisions, out of line: the straight code of the fast form has to stay small, the
+// warps of a CTA run it in different places and out of the instruction caches otherwise.
+template <int G>
+__device__ __noinline__ void walk_group_ieee(ObsGroup<G>* g, int i0, int span, const float* tile, int width, const float* square,
+                                             float s, int joint) {
+  const float* row[G];
+#pragma unroll
+  for (int c = 0; c < G; ++c) row[c] = tile + obs_row(i0 + c, width);
+  walk_group<G, false>(*g, i0, span, row, nullptr, square + i0, nullptr, s, 0.f, 0.f, joint);
+}
+
 // One column block [start, start+width).  Bound by the dependent chain of a column.  All four lanes of
 // a row walk it together in registers, a group at a time (the reciprocals of the divisors are made
 // once, which turns a division into five dependent multiply-adds), and they share the update of the
 // columns still open, group by group, 16 bytes at a time in the packed form of two.  Eight lanes per row,
 // a division in each step of the chain and an update of all open columns per column: 161 us per block of
-// 192 columns, 9216 rows; now 101 us.
+// 192 columns, 9216 rows; four lanes and groups with the IEEE division inline 101 us; out of line 86 us.
 // Shared memory: factor tile, three reciprocal rows, then per row two float rows (open values, which
 // become the finalised ones, and errors), then a byte per group and row (its selected zeros).
 template <int G>
@@ -95,7 +177,6 @@ obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start
     in_range = in_range && within(d, 0x1p-15f, 0x1p15f);
   }
   const bool exact = __syncthreads_and(in_range);
-  const float inf = __int_as_float(0x7f800000);
   float* open = open_all + slot * pitch;
   float* err = err_all + slot * pitch;
   uint8_t* chosen = chosen_all + slot * groups;
@@ -118,46 +199,24 @@ obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start
     __syncwarp();
     for (int group = 0; group < groups; ++group) {
       const int i0 = group * G, span = min(G, width - i0);
-      float v[G], e[G];
+      const float* frow[G];
 #pragma unroll
-      for (int c = 0; c < G; ++c) v[c] = c < span ? open[i0 + c] : 0.f;
-      // the two smallest scores (one or none in an incomplete group), ties to the lower column
-      const int remove = max(0, 2 - (G - span));
-      float low = inf, next = inf;
-      int first = G, second = G;
+      for (int c = 0; c < G; ++c) frow[c] = tile + obs_row(i0 + c, width);
+      ObsGroup<G> g;
 #pragma unroll
-      for (int c = 0; c < G; ++c) {
-        if (c < span) {
-          const float vv = __fmul_rn(v[c], v[c]);
-          const float score = exact && (vv == 0.f || within(vv, 0x1p-90f, 0x1p60f)) ? quotient(vv, square[i0 + c], square_recip[i0 + c])
-                                                              : __fdiv_rn(vv, square[i0 + c]);
-          if (first == G || score < low) { next = low; second = first; low = score; first = c; }
-          else if (second == G || score < next) { next = score; second = c; }
-        }
+      for (int c = 0; c < G; ++c) g.v[c] = c < span ? open[i0 + c] : 0.f;
+      g.loss = loss;
+      bool ok = exact;
+      if (ok) ok = walk_group<G, true>(g, i0, span, frow, recip + i0, square + i0, square_recip + i0, s, s_recip, v_limit, joint);
+      if (!ok) {
+        ObsGroup<G> again;
+#pragma unroll
+        for (int c = 0; c < G; ++c) again.v[c] = c < span ? open[i0 + c] : 0.f;
+        again.loss = loss;
+        walk_group_ieee<G>(&again, i0, span, tile, width, square, s, joint);
+        g = again;
       }
-      const unsigned mask = (remove > 0 ? 1u << first : 0u) | (remove > 1 ? 1u << second : 0u);
-#pragma unroll
-      for (int c = 0; c < G; ++c) {
-        e[c] = 0.f;
-        if (c < span) {
-          const float* frow = tile + obs_row(i0 + c, width) + i0;      // frow[d] = factor[i0 + c][i0 + d]
-          float fin = v[c];
-          if (joint) {
-            float g;
-            if (fabsf(v[c]) <= v_limit) g = fminf(127.f, fmaxf(-128.f, copysignf(rintf(quotient(v[c], s, s_recip)), v[c])));
-            else g = round_to_grid(v[c], s);
-            fin = __fmul_rn(g, s);
-          }
-          if (mask >> c & 1u) fin = 0.f;
-          const float d = __fsub_rn(v[c], fin);
-          if (exact && within(d, 0x1p-90f, 0x1p60f)) e[c] = quotient(d, frow[c], recip[i0 + c]);
-          else e[c] = exact && d == 0.f ? __fmul_rn(d, recip[i0 + c]) : __fdiv_rn(d, frow[c]);
-          loss = __fadd_rn(loss, __fmul_rn(__fmul_rn(e[c], e[c]), 0.5f));
-          v[c] = fin;
-#pragma unroll
-          for (int o = c + 1; o < G; ++o) v[o] = __fsub_rn(v[o], __fmul_rn(e[c], frow[o]));
-        }
-      }
+      loss = g.loss;
       // The group's errors on the open columns: o = (o - e0 f0) - e1 f1 ..., two columns at a time.  The
       // packed multiply and add of sm_100a are contracted to one rounding whatever their rounding
       // modifiers say, so the product is made by a multiply-add onto a -0 that the compiler does not know
@@ -165,13 +224,9 @@ obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start
       const float2 none = make_float2(minus_zero, minus_zero);
       const int i1 = i0 + G;
       if (i1 < width) {
-        const float* frow[G];
         float2 minus[G];
 #pragma unroll
-        for (int c = 0; c < G; ++c) {
-          frow[c] = tile + obs_row(i0 + c, width);
-          minus[c] = make_float2(-e[c], -e[c]);
-        }
+        for (int c = 0; c < G; ++c) minus[c] = make_float2(-g.e[c], -g.e[c]);
         if (G == 6 && (i1 & 2) && sl == 0) {
           float2 o = *reinterpret_cast<float2*>(open + i1);
 #pragma unroll
@@ -199,8 +254,8 @@ obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start
       __syncwarp();                   // every lane of the row has read the group's values
 #pragma unroll
       for (int c = 0; c < G; ++c)
-        if (sl == (c & (kLanesPerRow - 1)) && c < span) { open[i0 + c] = v[c]; err[i0 + c] = e[c]; }
-      if (sl == 0) chosen[group] = static_cast<uint8_t>(mask);
+        if (sl == (c & (kLanesPerRow - 1)) && c < span) { open[i0 + c] = g.v[c]; err[i0 + c] = g.e[c]; }
+      if (sl == 0) chosen[group] = static_cast<uint8_t>(g.mask);
       __syncwarp();
     }
     if (sl == 0 && row < rows) losses[row] = loss;
@@ -220,16 +275,17 @@ obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start
 
 // w[r, stop + j] -= sum_k errors[r, k] * upper[start + k, stop + j], the sum taken as
 // acc = fma(e, u, acc) from acc = 0 in increasing k.  Bound by the FP32 pipes and, next to them, the
-// shared-memory port: 128 x 128 output tile, 8 x 16 per thread (rows ty*4+i and 64+ty*4+i, columns
-// 32*h+tx*4+j) in the packed form of two multiply-adds, so that six 16-byte reads feed 64 of them.  Two
+// shared-memory port: 128 x 96 output tile (blocks are 192 wide), 8 x 12 per thread (rows ty*4+i and 64+ty*4+i,
+// columns 32*h+tx*4+j) in the packed form of two multiply-adds, so that five 16-byte reads feed 48 of them.  Two
 // slabs: the next one's B comes in by asynchronous copies, its A through registers, while the current one
 // is multiplied.  VEC: 16-byte accesses of the factor, the errors and w (all rows 16-byte aligned).
 // 8 x 8 per thread, scalar multiply-adds, scalar loads, one slab: 202 us a block (26 TFLOP/s) at 9216 x
-// 3072 in blocks of 192; packed multiply-adds and two slabs alone 174 us; this form 148 us.
-constexpr int kTileM = 128, kTileN = 128, kTileK = 16;
+// 3072 in blocks of 192; packed multiply-adds and two slabs alone 174 us; 8 x 16 per thread
+// on 128 x 128 tiles, two CTAs per SM, 148 us; this form, three CTAs per SM, 130 us.
+constexpr int kTileM = 128, kTileN = 96, kTileK = 16, kQuads = kTileN / 32;
 
 template <bool VEC>
-__global__ void __launch_bounds__(128, 2)
+__global__ void __launch_bounds__(128, 3)
 obs_trailing_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start, int width,
                     const float* __restrict__ upper, const float* __restrict__ errors) {
   __shared__ __align__(16) float a_s[2][kTileK][kTileM];
@@ -263,7 +319,7 @@ obs_trailing_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t st
     const bool k_ok = k0 + ty < width;
     const float* src = upper + (start + (k_ok ? k0 + ty : 0)) * columns + stop;
 #pragma unroll
-    for (int h = 0; h < 4; ++h)
+    for (int h = 0; h < kQuads; ++h)
 #pragma unroll
       for (int j = 0; j < 4; j += VEC ? 4 : 1) {
         const int c = 32 * h + tx * 4 + j;
@@ -273,11 +329,11 @@ obs_trailing_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t st
         else ptx::cp_async4(&b_s[slab][ty][c], from, in ? 4u : 0u);
       }
   };
-  float2 acc[8][8];
+  float2 acc[8][2 * kQuads];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    for (int j = 0; j < 2 * kQuads; ++j) acc[i][j] = make_float2(0.f, 0.f);
   fetch_a(0);
   fetch_b(0, 0);
   store_a(0);
@@ -289,9 +345,9 @@ obs_trailing_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t st
     if (more) { fetch_b(k0 + kTileK, slab ^ 1); fetch_a(k0 + kTileK); }
 #pragma unroll
     for (int k = 0; k < kTileK; ++k) {
-      float2 b[8];
+      float2 b[2 * kQuads];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
+      for (int h = 0; h < kQuads; ++h) {
         const float4 v = *reinterpret_cast<const float4*>(&b_s[slab][k][32 * h + tx * 4]);
         b[2 * h] = make_float2(v.x, v.y);
         b[2 * h + 1] = make_float2(v.z, v.w);
@@ -303,7 +359,7 @@ obs_trailing_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t st
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[4 * h + i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[4 * h + i][j]);
+          for (int j = 0; j < 2 * kQuads; ++j) acc[4 * h + i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[4 * h + i][j]);
       }
     }
     if (more) {
@@ -318,7 +374,7 @@ obs_trailing_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t st
     if (r >= rows) continue;
     float* wr = w + static_cast<int64_t>(r) * columns + stop;
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
+    for (int h = 0; h < kQuads; ++h) {
       const int c = col0 + 32 * h + tx * 4;
       const float2 lo = acc[i][2 * h], hi = acc[i][2 * h + 1];
       if constexpr (VEC) {
