@@ -175,10 +175,12 @@ DeviceInfo* device_info() {
 // Token tile of a launch (256 channels x NT tokens per cluster): the candidate with the smallest
 // rounds x cost-per-tile; ties go to the smaller tile.  Cost of one tile in cycles = blocks of 128
 // lifted columns x per-block cost + per-tile cost, both fitted per token tile (relative least
-// squares) to GEMM times measured by CUDA-graph replay over 23 shapes of the benchmark
-// configurations (K' 1152 .. 18432, M 256 .. 16384).  The per-tile part is the pipeline fill, the
-// epilogue tail and the barrier round trips; 256 has a single accumulator, so its epilogue is
-// exposed.  Over those shapes the model's choice costs 0.4 % more than the best tile per shape.
+// squares, with a constant of 8463 cycles per launch that does not matter to the choice) to GEMM times
+// measured by CUDA-graph replay over 24 shapes (K' 1024 .. 18432, M 64 .. 16384, weights read from HBM).
+// The per-tile part is the epilogue tail and the barrier round trips; 256 has a single accumulator, so
+// its epilogue is exposed.  On 26 other shapes (K' 512 .. 16000, M 128 .. 16384) the choice costs 0.2 % more
+// than the best tile per shape, 3.4 % at worst; the constants fitted to the MMA loop with a metadata warp
+// cost 2.1 % there, 12.5 % at worst (4096 x 1152 -> 4608 streaming: 18.2 us, now 16.2).
 std::atomic<long long> g_split_launches{0};
 
 // The split schedule's area of `stream`, handed out now if `create` and one is left (the pool is
@@ -243,8 +245,8 @@ DeviceInfo::SplitArea* split_workspace(DeviceInfo* dev, cudaStream_t stream, boo
 }
 
 constexpr int kTiles[kTileCount] = {128, 192, 224, 240, 256};
-constexpr double kPerBlock[kTileCount] = {351.0, 415.0, 414.0, 425.0, 448.0};
-constexpr double kPerTile[kTileCount] = {2477.0, 2813.0, 4107.0, 3925.0, 5799.0};
+constexpr double kPerBlock[kTileCount] = {252.0, 331.0, 344.0, 351.0, 382.0};
+constexpr double kPerTile[kTileCount] = {759.0, 1098.0, 1563.0, 1726.0, 2058.0};
 
 // Split schedule (see Walk in ss_gemm_pair.cuh): the clusters share the tiles x stages evenly, so a
 // launch costs tiles / clusters (not rounded up) tile costs, plus what the shared tiles cost: every
