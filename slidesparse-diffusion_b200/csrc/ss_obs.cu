@@ -52,15 +52,17 @@ struct ObsGroup {
 
 // Walks a group: the two smallest scores (one or none in an incomplete group, ties to the lower column)
 // are selected, then column by column it is rounded, its error taken and the group's later columns
-// updated.  FAST divides by the reciprocals and returns whether every division was within their range.
-template <int G, bool FAST>
+// updated.  FAST takes complete groups only, divides by the reciprocals and returns whether every division
+// was within their range: straight code without a branch, so that the loads of all columns go out first.
+template <int G, bool JOINT, bool FAST>
 __device__ __forceinline__ bool walk_group(ObsGroup<G>& g, int i0, int span, const float* const (&row)[G], const float* recip,
                                            const float* square, const float* square_recip, float s, float s_recip,
-                                           float v_limit, int joint) {
+                                           float v_limit) {
   bool ok = true;
+  if constexpr (FAST) span = G;
   const int remove = max(0, 2 - (G - span));
   float low = 0.f, next = 0.f;
-  int first = G, second = G;
+  int first = 0, second = 0;
 #pragma unroll
   for (int c = 0; c < G; ++c) {
     if (c < span) {
@@ -72,8 +74,13 @@ __device__ __forceinline__ bool walk_group(ObsGroup<G>& g, int i0, int span, con
       } else {
         score = __fdiv_rn(vv, square[c]);
       }
-      if (first == G || score < low) { next = low; second = first; low = score; first = c; }
-      else if (second == G || score < next) { next = score; second = c; }
+      if (c == 0) {
+        low = score;
+      } else if (score < low) {
+        next = low; second = first; low = score; first = c;
+      } else if (c == 1 || score < next) {
+        next = score; second = c;
+      }
     }
   }
   g.mask = (remove > 0 ? 1u << first : 0u) | (remove > 1 ? 1u << second : 0u);
@@ -81,17 +88,20 @@ __device__ __forceinline__ bool walk_group(ObsGroup<G>& g, int i0, int span, con
   for (int c = 0; c < G; ++c) {
     g.e[c] = 0.f;
     if (c < span) {
-      const float* frow = row[c] + i0;                 // frow[o] = factor[i0 + c][i0 + o]
+      float frow[G];                                   // frow[o] = factor[i0 + c][i0 + o] for o >= c
+#pragma unroll
+      for (int o = c & ~1; o < G; o += 2) {
+        const float2 f = *reinterpret_cast<const float2*>(row[c] + i0 + o);
+        frow[o] = f.x;
+        frow[o + 1] = f.y;
+      }
       float fin = g.v[c];
-      if (joint) {
-        float q;
-        if constexpr (FAST) {
-          q = fminf(127.f, fmaxf(-128.f, copysignf(rintf(quotient(g.v[c], s, s_recip)), g.v[c])));
-          ok = ok && fabsf(g.v[c]) <= v_limit;
-        } else {
-          q = round_to_grid(g.v[c], s);
-        }
+      if constexpr (JOINT && FAST) {
+        const float q = fminf(127.f, fmaxf(-128.f, copysignf(rintf(quotient(g.v[c], s, s_recip)), g.v[c])));
+        ok = ok && fabsf(g.v[c]) <= v_limit;
         fin = __fmul_rn(q, s);
+      } else if constexpr (JOINT) {
+        fin = __fmul_rn(round_to_grid(g.v[c], s), s);
       }
       if (g.mask >> c & 1u) fin = 0.f;
       const float d = __fsub_rn(g.v[c], fin);
@@ -125,13 +135,13 @@ __host__ __device__ __forceinline__ int obs_tile_floats(int width) { return obs_
 
 // The same with IEEE divisions, out of line: the straight code of the fast form has to stay small, the
 // warps of a CTA run it in different places and out of the instruction caches otherwise.
-template <int G>
+template <int G, bool JOINT>
 __device__ __noinline__ void walk_group_ieee(ObsGroup<G>* g, int i0, int span, const float* tile, int width, const float* square,
-                                             float s, int joint) {
+                                             float s) {
   const float* row[G];
 #pragma unroll
   for (int c = 0; c < G; ++c) row[c] = tile + obs_row(i0 + c, width);
-  walk_group<G, false>(*g, i0, span, row, nullptr, square + i0, nullptr, s, 0.f, 0.f, joint);
+  walk_group<G, JOINT, false>(*g, i0, span, row, nullptr, square + i0, nullptr, s, 0.f, 0.f);
 }
 
 // One column block [start, start+width).  Bound by the dependent chain of a column.  All four lanes of
@@ -139,13 +149,14 @@ __device__ __noinline__ void walk_group_ieee(ObsGroup<G>* g, int i0, int span, c
 // once, which turns a division into five dependent multiply-adds), and they share the update of the
 // columns still open, group by group, 16 bytes at a time in the packed form of two.  Eight lanes per row,
 // a division in each step of the chain and an update of all open columns per column: 161 us per block of
-// 192 columns, 9216 rows; four lanes and groups with the IEEE division inline 101 us; out of line 86 us.
+// 192 columns, 9216 rows; four lanes and groups with the IEEE division inline 101 us; out of line 86 us;
+// complete groups in code without branches 74 us.
 // Shared memory: factor tile, three reciprocal rows, then per row two float rows (open values, which
 // become the finalised ones, and errors), then a byte per group and row (its selected zeros).
-template <int G>
+template <int G, bool JOINT>
 __global__ void __launch_bounds__(kObsMaxRows * kLanesPerRow, 1)
 obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start, int width, int rows_per_cta,
-                 const float* __restrict__ upper, const float* __restrict__ scales, int joint, float minus_zero,
+                 const float* __restrict__ upper, const float* __restrict__ scales, float minus_zero,
                  uint8_t* __restrict__ zeros, float* __restrict__ errors, float* __restrict__ losses) {
   extern __shared__ __align__(16) unsigned char smem[];
   float* tile = reinterpret_cast<float*>(smem);
@@ -206,14 +217,14 @@ obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start
 #pragma unroll
       for (int c = 0; c < G; ++c) g.v[c] = c < span ? open[i0 + c] : 0.f;
       g.loss = loss;
-      bool ok = exact;
-      if (ok) ok = walk_group<G, true>(g, i0, span, frow, recip + i0, square + i0, square_recip + i0, s, s_recip, v_limit, joint);
+      bool ok = exact && span == G;
+      if (ok) ok = walk_group<G, JOINT, true>(g, i0, span, frow, recip + i0, square + i0, square_recip + i0, s, s_recip, v_limit);
       if (!ok) {
         ObsGroup<G> again;
 #pragma unroll
         for (int c = 0; c < G; ++c) again.v[c] = c < span ? open[i0 + c] : 0.f;
         again.loss = loss;
-        walk_group_ieee<G>(&again, i0, span, tile, width, square, s, joint);
+        walk_group_ieee<G, JOINT>(&again, i0, span, tile, width, square, s);
         g = again;
       }
       loss = g.loss;
@@ -282,6 +293,7 @@ obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start
 // 8 x 8 per thread, scalar multiply-adds, scalar loads, one slab: 202 us a block (26 TFLOP/s) at 9216 x
 // 3072 in blocks of 192; packed multiply-adds and two slabs alone 174 us; 8 x 16 per thread
 // on 128 x 128 tiles, two CTAs per SM, 148 us; this form, three CTAs per SM, 130 us.
+// (Half a slab of A in registers, 128 x 64 tiles with four CTAs: 133 us; two CTAs of this tile: 140 us.)
 constexpr int kTileM = 128, kTileN = 96, kTileK = 16, kQuads = kTileN / 32;
 
 template <bool VEC>
@@ -469,10 +481,12 @@ extern "C" int ss_obs_block(float* w, int64_t rows, int64_t columns, int64_t sta
   const size_t smem = obs_block_smem(wide, group, static_cast<int>(per_cta));
   const int64_t wanted = (rows + per_cta - 1) / per_cta;
   const unsigned grid = static_cast<unsigned>(wanted < sms ? wanted : sms);
-  auto kernel = group == 4 ? obs_block_kernel<4> : group == 6 ? obs_block_kernel<6> : obs_block_kernel<8>;
+  auto kernel = group == 4 ? (joint ? obs_block_kernel<4, true> : obs_block_kernel<4, false>)
+              : group == 6 ? (joint ? obs_block_kernel<6, true> : obs_block_kernel<6, false>)
+                           : (joint ? obs_block_kernel<8, true> : obs_block_kernel<8, false>);
   SS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   kernel<<<grid, static_cast<unsigned>(per_cta) * kLanesPerRow, smem, static_cast<cudaStream_t>(stream)>>>(
-      w, static_cast<int>(rows), columns, start, wide, static_cast<int>(per_cta), upper, scales, joint != 0, -0.0f, zeros,
+      w, static_cast<int>(rows), columns, start, wide, static_cast<int>(per_cta), upper, scales, -0.0f, zeros,
       errors, losses);
   SS_CUDA(cudaGetLastError());
   return SS_OK;
