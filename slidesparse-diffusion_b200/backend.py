@@ -544,10 +544,10 @@ def quantize_lift_fused(input, group, prologue):
 
 def gate_add(x, gate, y):
     """x + gate[:, None] * y with BF16 x, y [batch, rows, n] and gate [batch, n]: one kernel where the
-    library is loaded and nothing has to be differentiated or traced, torch.addcmul otherwise."""
-    if (_ops_registered and x.is_cuda and x.dtype == y.dtype == gate.dtype == torch.bfloat16
-            and not (torch.is_grad_enabled() and (x.requires_grad or y.requires_grad or gate.requires_grad))
-            and not torch.compiler.is_compiling()):
+    library is loaded and plain tensors are at hand (the operator itself leaves gradients, tangents and
+    batching to torch), torch.addcmul otherwise."""
+    if (not torch.compiler.is_compiling() and _ops_registered and type(x) is type(y) is type(gate) is torch.Tensor
+            and x.is_cuda and x.dtype == y.dtype == gate.dtype == torch.bfloat16):
         return torch.ops.slidesparse_b200.gate_add(x, gate, y)
     return torch.addcmul(x, gate[:, None], y)
 
@@ -809,7 +809,7 @@ def _register_ops(binding):
         for name in ("projection", "projection_packed16", "projection_scalar"):
             mild.impl(name, _projection, "CUDA")
         prepared.impl("run", _prepared_run, "CUDA")
-        own.impl("gate_add", lambda x, gate, y: torch.addcmul(x, gate[:, None], y), "CUDA")
+        own.impl("gate_add", lambda x, gate, y: torch.addcmul(x, gate[:, None], y), "CompositeImplicitAutograd")
         own.impl("projection_fused", _op_fused, "CUDA")
         own.impl("projection_fused_accumulate_", _op_fused_accumulate, "CUDA")
     _libraries.append(own)
@@ -818,9 +818,10 @@ def _register_ops(binding):
     def _fake_fused(input, prologue, shift, scale, eps, packed, metadata, scales, bias, group, n, output_addend=None):
         return input.new_empty((*input.shape[:-1], n))
 
-    @torch.library.register_fake("slidesparse_b200::gate_add")
-    def _fake_gate_add(x, gate, y):
-        return torch.empty_like(x)
+    if binding is not None:                   # the other form is made of torch operators
+        @torch.library.register_fake("slidesparse_b200::gate_add")
+        def _fake_gate_add(x, gate, y):
+            return torch.empty_like(x)
 
     @torch.library.register_fake("slidesparse_b200::projection_fused_accumulate_")
     def _fake_fused_accumulate(residual, input, prologue, shift, scale, eps, packed, metadata, scales, bias, group, n, gate):

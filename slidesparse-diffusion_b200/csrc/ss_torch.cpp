@@ -294,6 +294,20 @@ void projection_fused_accumulate(const Tensor& residual, const Tensor& input, in
   projection_fused_into(input, prologue, shift, scale, eps, packed, metadata, scales, bias, group, n, std::nullopt, &gate, out);
 }
 
+// x + gate[:, None] * y in torch's own operators, which have every derivative and batching rule
+Tensor gate_add_torch(const Tensor& x, const Tensor& gate, const Tensor& y) { return at::addcmul(x, gate.unsqueeze(1), y); }
+
+// Where a gradient or a forward-mode tangent hangs on an operand (a dual tensor does not require gradients),
+// torch's operators; the kernel knows neither.
+Tensor gate_add_autograd(const Tensor& x, const Tensor& gate, const Tensor& y) {
+  for (const Tensor* t : {&x, &gate, &y})
+    if ((at::GradMode::is_enabled() && t->requires_grad()) || t->_fw_grad(/*level=*/0).defined()) return gate_add_torch(x, gate, y);
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("slidesparse_b200::gate_add", "")
+                             .typed<Tensor(const Tensor&, const Tensor&, const Tensor&)>();
+  const at::AutoDispatchBelowADInplaceOrView below;
+  return op.call(x, gate, y);
+}
+
 // x + gate[:, None] * y: one pass of this library's kernel where the rows allow it, torch's otherwise
 Tensor gate_add(const Tensor& x, const Tensor& gate, const Tensor& y) {
   auto aligned = [](const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
@@ -303,7 +317,7 @@ Tensor gate_add(const Tensor& x, const Tensor& gate, const Tensor& y) {
                       x.is_contiguous() && y.is_contiguous() && x.size(2) % 8 == 0 && gate.stride(1) == 1 &&
                       (gate.size(0) == 1 || (gate.stride(0) % 8 == 0 && gate.stride(0) >= gate.size(1))) &&
                       aligned(x) && aligned(y) && aligned(gate) && x.size(0) * x.size(1) < (1ll << 31) && x.size(2) < (1ll << 31);
-  if (!usable) return at::addcmul(x, gate.unsqueeze(1), y);
+  if (!usable) return gate_add_torch(x, gate, y);
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor out = new_output(x, x.size(2));
   check(ss_gate_add(x.data_ptr(), gate.data_ptr(), gate.size(0) > 1 ? gate.stride(0) : gate.size(1), y.data_ptr(), out.data_ptr(),
@@ -332,3 +346,7 @@ TORCH_LIBRARY_IMPL(slidesparse_b200, CUDA, m) {
   m.impl("projection_fused_accumulate_", TORCH_FN(projection_fused_accumulate));
   m.impl("gate_add", TORCH_FN(gate_add));
 }
+
+TORCH_LIBRARY_IMPL(slidesparse_b200, Autograd, m) { m.impl("gate_add", TORCH_FN(gate_add_autograd)); }
+
+TORCH_LIBRARY_IMPL(slidesparse_b200, FuncTorchBatched, m) { m.impl("gate_add", TORCH_FN(gate_add_torch)); }
