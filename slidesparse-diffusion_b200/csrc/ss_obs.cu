@@ -35,8 +35,9 @@ __device__ __forceinline__ float round_to_grid(float v, float s) {
   return fminf(127.f, fmaxf(-128.f, rintf(__fdiv_rn(v, s))));
 }
 
-// Ranges in which quotient() is exact: divisors 2^-15 .. 2^15 (their squares 2^-30 .. 2^30), scales
-// 2^-60 .. 2^60, dividends +0 and 2^-90 .. 2^60.  Outside (and for NaN) the IEEE division runs.
+// Ranges in which quotient() is exact: divisors 2^-15 .. 2^15 (their squares 2^-30 .. 2^30), positive scales
+// 2^-60 .. 2^60 (the rounded quotient takes the dividend's sign), dividends +0 and 2^-90 .. 2^60.  Outside
+// (and for NaN) the IEEE division runs.
 __device__ __forceinline__ bool within(float v, float lo, float hi) { return fabsf(v) >= lo && fabsf(v) <= hi; }
 __device__ __forceinline__ bool dividend_ok(float v) {
   const uint32_t bits = __float_as_uint(v), lo = (127u - 90u) << 23, hi = (127u + 60u) << 23;
@@ -204,7 +205,7 @@ obs_block_kernel(float* __restrict__ w, int rows, int64_t columns, int64_t start
     }
     const float s = row < rows ? scales[row] : 1.f;
     const float s_recip = __fdiv_rn(1.f, s);
-    const float v_limit = within(s, 0x1p-60f, 0x1p60f) ? 0x1p60f : -1.f;
+    const float v_limit = s >= 0x1p-60f && s <= 0x1p60f ? 0x1p60f : -1.f;
     float loss = row < rows ? losses[row] : 0.f;
     ptx::cp_async_wait_all();
     __syncwarp();

@@ -7,6 +7,8 @@ import numpy as np
 import pytest
 import torch
 
+from gpu_util import check, ptr, stream
+
 pytestmark = pytest.mark.gpu
 GOLDEN = np.load(Path(__file__).resolve().parent / "golden" / "reconstruction.npz")
 CASES = [tuple(int(v) for v in row) for row in GOLDEN["cases"]]
@@ -189,3 +191,24 @@ def test_kernels_match_the_oracle_at_the_edges(recon, oracle_c, rows, columns, g
     assert np.array_equal(result["qweight"].cpu().numpy(), q)
     assert np.array_equal(_bits(result["compensated"]), w.view(np.uint32))
     assert np.array_equal(_bits(result["proxy_loss"]), losses.view(np.uint32))
+
+
+@pytest.mark.parametrize("group", [4, 6, 8])
+def test_block_entry_takes_scales_of_either_sign(recon, backend, oracle_c, group):
+    """The C entry states no sign for the scales: a negative one rounds v / s like a positive one does."""
+    rows, columns = 24, 96
+    weight, hessian = _synthetic(rows, columns, seed=group)
+    curvature = recon.factor_hessian(hessian)
+    scales = recon.channel_scales(weight).clone()
+    scales[::2] *= -1
+    _, zeros, w, losses = oracle_c.obs_compress(weight.numpy(), curvature.upper.numpy(), curvature.dead.numpy(),
+                                                scales.numpy(), group, columns, True)
+    dev = "cuda:0"
+    on_gpu = [weight.to(dev).contiguous(), curvature.upper.to(dev).contiguous(), scales.to(dev)]
+    got_zeros = torch.zeros(rows, columns, dtype=torch.uint8, device=dev)
+    errors, got_losses = torch.zeros(rows, columns, device=dev), torch.zeros(rows, device=dev)
+    check(backend, backend.library().ss_obs_block(ptr(on_gpu[0]), rows, columns, 0, columns, ptr(on_gpu[1]), ptr(on_gpu[2]), group, 1,
+                                                  ptr(got_zeros), ptr(errors), ptr(got_losses), stream()))
+    assert np.array_equal(got_zeros.cpu().numpy().astype(bool), zeros.astype(bool))
+    assert np.array_equal(_bits(on_gpu[0]), w.view(np.uint32))
+    assert np.array_equal(_bits(got_losses), losses.view(np.uint32))
