@@ -85,3 +85,14 @@ def test_widest_block_is_reported_without_a_gpu(recon):
     assert recon.max_blocksize() == 225
     with pytest.raises(ValueError):
         recon.compress(torch.randn(3, 12), recon.factor_hessian(torch.eye(12)), 4, blocksize=228)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32, torch.float16, torch.bfloat16, torch.float8_e4m3fn,
+                                   torch.float8_e5m2, torch.int8, torch.uint8, torch.bool])
+def test_channel_scales_of_every_element_type(recon, dtype):
+    """2 * absmax / 255 of the fp32 image of each row, whatever the weight is stored in."""
+    weight = (torch.randn(5, 40, generator=torch.Generator().manual_seed(1)) * 3).to(dtype)
+    weight[2] = torch.zeros(40, dtype=dtype)
+    image = weight.float().abs().amax(dim=1)
+    expect = torch.where(image > 0, 2 * image / torch.full_like(image, 255), torch.ones_like(image))
+    assert torch.equal(recon.channel_scales(weight), expect)
