@@ -331,6 +331,25 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // call grid_dep_wait before touching anything that kernel writes.  Both are no-ops otherwise.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Loads for what the overlapped kernel may have written.  __ldg (and a const __restrict__ pointer) allows
+// ld.global.nc, which is for data that nobody writes while this kernel lives, and it lives before
+// grid_dep_wait; these are ordinary loads, and as volatile statements they stay behind that wait.
+__device__ __forceinline__ uint4 ld_global(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ float ld_global(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_global(const uint16_t* p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
 __device__ __forceinline__ void tc_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }

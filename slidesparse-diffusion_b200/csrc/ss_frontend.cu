@@ -124,7 +124,7 @@ __device__ __forceinline__ void lift_chunk(const uint32_t* qw, uint32_t* ow) {
 // L: group size (4, 6, 8).  VEC: rows are 16-byte aligned and k % 8 == 0.  PRO: prologue (VEC only).
 template <int L, bool VEC, int PRO = kProNone>
 __global__ void __launch_bounds__(kMaxThreads)
-quant_lift_kernel(const uint16_t* __restrict__ x, int64_t sx, int8_t* __restrict__ q,
+quant_lift_kernel(const uint16_t* x, int64_t sx, int8_t* __restrict__ q,
                   float* __restrict__ sa, int m, int k, int pk, int nvec, int nchunks, const Prologue pro) {
   constexpr int CV = Chunk<L>::kVec, OW = Chunk<L>::kOutWords, kChunks = kMaxVec / CV;
   __shared__ uint32_t warp_max[kMaxThreads / 32];
@@ -152,13 +152,13 @@ quant_lift_kernel(const uint16_t* __restrict__ x, int64_t sx, int8_t* __restrict
       uint4 w = make_uint4(0u, 0u, 0u, 0u);
       if (live && idx < nvec) {
         if constexpr (VEC) {
-          w = __ldg(reinterpret_cast<const uint4*>(xr) + idx);
+          w = ptx::ld_global(reinterpret_cast<const uint4*>(xr) + idx);
         } else {
           uint32_t e[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int col = idx * 8 + j;
-            e[j] = col < k ? static_cast<uint32_t>(__ldg(xr + col)) : 0u;
+            e[j] = col < k ? ptx::ld_global(xr + col) : 0u;
           }
           w = make_uint4(e[0] | (e[1] << 16), e[2] | (e[3] << 16), e[4] | (e[5] << 16), e[6] | (e[7] << 16));
         }
@@ -217,7 +217,7 @@ quant_lift_kernel(const uint16_t* __restrict__ x, int64_t sx, int8_t* __restrict
         const int idx = (t + i * T) * CV + c;
         if (live && idx < nvec) {
           uint4& w = v[i][c];
-          const uint4 sh = __ldg(shift + idx), sc = __ldg(scale + idx);
+          const uint4 sh = ptx::ld_global(shift + idx), sc = ptx::ld_global(scale + idx);
           uint32_t e[4] = {w.x, w.y, w.z, w.w};
           const uint32_t hs[4] = {sh.x, sh.y, sh.z, sh.w}, cs[4] = {sc.x, sc.y, sc.z, sc.w};
 #pragma unroll
@@ -336,14 +336,14 @@ int launch_one(const void* x, int64_t sx, int m, int k, int pm, int pk, int8_t* 
 // exact in FP32, so one multiply-add rounds as multiply and add do.  Bound by HBM or L2; 2048 x 1152 behind
 // the attention of a block: torch's addcmul with the broadcast gate takes 8.9 us there.
 __global__ void __launch_bounds__(256)
-gate_add_kernel(const uint4* __restrict__ x, const uint16_t* __restrict__ gate, int64_t gate_stride,
-                const uint4* __restrict__ y, uint4* __restrict__ out, int64_t rows_per_batch, int vecs) {
+gate_add_kernel(const uint4* x, const uint16_t* gate, int64_t gate_stride, const uint4* y, uint4* out,
+                int64_t rows_per_batch, int vecs) {
   ptx::grid_dep_wait();
   ptx::grid_dep_launch();
   const int64_t row = blockIdx.x;
   const uint4* g = reinterpret_cast<const uint4*>(gate + row / rows_per_batch * gate_stride);
   for (int i = threadIdx.x; i < vecs; i += blockDim.x) {
-    const uint4 xv = __ldg(x + row * vecs + i), yv = __ldg(y + row * vecs + i), gv = __ldg(g + i);
+    const uint4 xv = ptx::ld_global(x + row * vecs + i), yv = ptx::ld_global(y + row * vecs + i), gv = ptx::ld_global(g + i);
     auto add = [](uint32_t a, uint32_t b, uint32_t c) { return pack_bf16(__ffma2_rn(unpack_bf16(b), unpack_bf16(c), unpack_bf16(a))); };
     out[row * vecs + i] = make_uint4(add(xv.x, gv.x, yv.x), add(xv.y, gv.y, yv.y), add(xv.z, gv.z, yv.z), add(xv.w, gv.w, yv.w));
   }

@@ -499,7 +499,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       const int pch = nxt.ch * (2 * kTileCh) + static_cast<int>(rank) * kTileCh + quad * 32 + lane_ch;
       const int ptok = nxt.tok * NT + half * 32 + lane;
 #pragma unroll
-      for (int i = 0; i < kMine; ++i) sa_next[i] = __ldg(args.sa + min(ptok + kPairSub * 32 * i, last_tok));
+      for (int i = 0; i < kMine; ++i) sa_next[i] = ptx::ld_global(args.sa + min(ptok + kPairSub * 32 * i, last_tok));
 #pragma unroll
       for (int i = 0; i < 4; ++i) sw_next[i] = __ldg(args.sw + min(pch + 8 * i, last_ch));   // channels lane_ch + 8 i
       if (args.bias) {
@@ -565,7 +565,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           const int tok = tok0 + c * 32 + 8 * j + (lane >> 2), ch = ch_w + 8 * (lane & 3);
           ad[j] = make_uint4(0u, 0u, 0u, 0u);
           if (tok < args.m && ch < args.n)
-            ad[j] = __ldg(reinterpret_cast<const uint4*>(args.addend + static_cast<long long>(tok) * args.addend_stride + ch));
+            ad[j] = ptx::ld_global(reinterpret_cast<const uint4*>(args.addend + static_cast<long long>(tok) * args.addend_stride + ch));
         }
       };
       if constexpr (ADDEND) {
@@ -835,7 +835,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       const int pch = nxt.ch * (2 * kTileCh) + static_cast<int>(rank) * kTileCh + quad * 32 + lane;
       const int ptok = nxt.tok * NT + half * 32 + lane;
 #pragma unroll
-      for (int i = 0; i < kMine; ++i) sa_next[i] = __ldg(args.sa + min(ptok + kPairSub * 32 * i, last_tok));
+      for (int i = 0; i < kMine; ++i) sa_next[i] = ptx::ld_global(args.sa + min(ptok + kPairSub * 32 * i, last_tok));
       sw_next = __ldg(args.sw + min(pch, last_ch));
       if (args.bias) bias_next = __ldg(args.bias + min(pch, last_ch));
     };
