@@ -223,10 +223,10 @@ int ss_micro_pair_rate(int64_t m, int64_t n, int64_t pk, int token_tile, int fla
                        double* cycles_per_stage, int64_t* stages);
 
 /* Diagnostic.  No counterpart in the reference.  Proves the exit path of the bounded waits without
- * starving a real kernel: one warp waits, for at most limit_ns (1 ns .. 100 ms), on an mbarrier
- * that nothing arrives on.  The wait must run out, the kernel must return normally and leave the
+ * starving a real kernel: a thread, then a whole warp, waits for at most limit_ns (1 ns .. 100 ms) on an
+ * mbarrier that nothing arrives on.  The waits must run out, the kernel must return normally and leave the
  * wait-limit bit (8) in the device status word, which the next ss_device_status reports (SS_E_DEVICE)
- * and clears; the context stays usable.  *elapsed_ns = how long the kernel actually waited.
+ * and clears; the context stays usable.  *elapsed_ns = how long the shorter of the two waits took.
  * Synchronises the device. */
 int ss_micro_wait_limit(int64_t limit_ns, int64_t* elapsed_ns);
 

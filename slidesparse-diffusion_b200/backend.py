@@ -444,8 +444,9 @@ def micro_pair_rate(m, n, pk, token_tile=0, no_mma=False, no_epilogue=False, no_
 
 
 def micro_wait_limit(limit_ns):
-    """Nanoseconds a kernel really waited on a barrier nobody signals before its bounded wait gave
-    up; leaves the wait-limit bit in the device status word (diagnostic)."""
+    """Nanoseconds a kernel really waited on a barrier nobody signals before its bounded waits (a
+    thread's, then a warp's: the shorter) gave up; leaves the wait-limit bit in the device status word
+    (diagnostic)."""
     elapsed = ctypes.c_int64()
     check(library().ss_micro_wait_limit(int(limit_ns), ctypes.byref(elapsed)))
     return elapsed.value

@@ -195,13 +195,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
 }
 
 // The same wait for a whole warp: the lanes leave together, by a vote, so that the compiler keeps what
-// follows on warp-uniform registers.
+// follows on warp-uniform registers.  Every lane has to have seen the phase complete, since any of them may
+// act on it and a vote orders no memory; none can miss it, as long as the barrier's next phase cannot
+// complete before this warp has acted (a ring's slot and its accumulators are such barriers).
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
                                                unsigned long long limit_ns = kDefaultWaitNs) {
-  if (__any_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
   uint64_t deadline = 0;
   for (uint32_t spin = 1;; ++spin) {
-    if (__any_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
     if ((spin & 0x3fu) == 0) {
       const uint64_t now = globaltimer_ns();
       if (deadline == 0) deadline = now + limit_ns;

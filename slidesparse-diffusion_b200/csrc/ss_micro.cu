@@ -104,17 +104,30 @@ int run_rate(int iters, int with_cp, double* cycles_per_mma) {
 namespace ss {
 namespace {
 
-// One warp waits, with the given limit, on an mbarrier that nothing ever arrives on.  The wait
-// must run out, the kernel must record that in the device status word and return normally.
+// A thread, then a whole warp, waits with the given limit on an mbarrier that nothing ever arrives on.  The
+// waits must run out, the kernel must record that in the device status word and return normally.  On a
+// barrier whose phase is complete the warp's wait must succeed at once.
 __global__ void wait_limit_kernel(unsigned long long limit_ns, uint32_t* status, unsigned long long* elapsed_ns) {
-  __shared__ uint64_t bar;
+  __shared__ uint64_t silent, done;
   if (threadIdx.x == 0) {
-    ptx::mbar_init(&bar, 1);
+    ptx::mbar_init(&silent, 1);
+    ptx::mbar_init(&done, 1);
     ptx::fence_barrier_init();
-    const uint64_t t0 = ptx::globaltimer_ns();
-    const bool arrived = ptx::mbar_wait(&bar, 0, limit_ns);
-    elapsed_ns[0] = ptx::globaltimer_ns() - t0;
-    if (!arrived) atomicOr(status, kStatusProbeTimeout);
+    ptx::mbar_arrive_expect_tx(&done, 0);
+  }
+  __syncwarp();
+  uint64_t t0 = ptx::globaltimer_ns(), waited = ~0ull;
+  if (threadIdx.x == 0) {
+    if (!ptx::mbar_wait(&silent, 0, limit_ns)) waited = ptx::globaltimer_ns() - t0;
+  }
+  __syncwarp();
+  t0 = ptx::globaltimer_ns();
+  const bool arrived = ptx::mbar_wait_warp(&silent, 0, limit_ns);
+  const uint64_t together = ptx::globaltimer_ns() - t0;
+  if (!ptx::mbar_wait_warp(&done, 0, limit_ns) && threadIdx.x == 0) atomicOr(status, kStatusMmaTimeout);
+  if (threadIdx.x == 0) {
+    elapsed_ns[0] = waited < together ? waited : together;
+    if (!arrived && waited != ~0ull) atomicOr(status, kStatusProbeTimeout);
   }
 }
 
