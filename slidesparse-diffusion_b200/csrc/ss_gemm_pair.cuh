@@ -634,14 +634,20 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         }
         __syncwarp();
         SS_PF(pe_prep);
-        // gated accumulation: the 32 tokens of a chunk belong to one batch (rows_per_batch % 32 == 0)
-        float gate[4] = {1.f, 1.f, 1.f, 1.f};
+        // gated accumulation: the 32 tokens of a chunk belong to one batch (rows_per_batch % 32 == 0), or,
+        // where tiles of 240 tokens start on an odd multiple of 16, each half of them does
+        constexpr int kGates = GATED && NT % 32 != 0 ? 2 : 1;
+        float gate[kGates][4] = {};
         if constexpr (GATED) {
-          const __nv_bfloat16* g = args.gate + static_cast<long long>((tok0 + c * 32) / args.rows_per_batch) * args.gate_stride;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int ch = ch_w + lane_ch + 8 * i;
-            gate[i] = ch < args.n ? __bfloat162float(g[ch]) : 0.f;
+          for (int t = 0; t < kGates; ++t) {
+            const int tok = min(tok0 + c * 32 + 16 * t, args.m - 1);
+            const __nv_bfloat16* g = args.gate + static_cast<long long>(tok / args.rows_per_batch) * args.gate_stride;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int ch = ch_w + lane_ch + 8 * i;
+              gate[t][i] = ch < args.n ? __bfloat162float(g[ch]) : 0.f;
+            }
           }
         }
         // this thread addresses row lane%8 of matrix lane/8 in every stmatrix.x4: matrices are
@@ -680,7 +686,10 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                 const float2 acc = make_float2(__int2float_rn(static_cast<int32_t>(r[2 * ab])),
                                                __int2float_rn(static_cast<int32_t>(r[2 * ab + 1])));
                 float2 y = __ffma2_rn(acc, __fmul2_rn(s, make_float2(w, w)), make_float2(b, b));
-                if constexpr (GATED) y = __fmul2_rn(make_float2(gate[2 * h + ab], gate[2 * h + ab]), y);
+                if constexpr (GATED) {
+                  const float gv = gate[gp & (kGates - 1)][2 * h + ab];
+                  y = __fmul2_rn(make_float2(gv, gv), y);
+                }
                 if constexpr (ADDEND) {
                   const uint32_t t = addend[2 * gi + ab];
                   y = make_float2(__fadd_rn(y.x, __uint_as_float(t << 16)), __fadd_rn(y.y, __uint_as_float(t & 0xffff0000u)));

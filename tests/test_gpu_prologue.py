@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import bits
+from gpu_util import bits, option
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -138,6 +138,27 @@ def test_gated_accumulation_matches_oracle(sdk, backend, oracle, oracle_c, mode,
     # the same through the PyTorch operators, within BF16 rounding of the intermediate
     eager = torch.addcmul(residual.to(DEV), wide.to(DEV)[:, 2 * n:3 * n][:, None], op(x.to(DEV)))
     assert float((eager.float() - out.float()).abs().max()) <= 0.02 * float(eager.float().abs().max())
+
+
+@pytest.mark.parametrize("tile", [0, 128, 192, 224, 240, 256])
+@pytest.mark.parametrize("batch,rows", [(2, 256), (17, 32), (3, 480), (5, 224)])
+def test_gate_of_every_batch_in_every_tile(sdk, backend, oracle, oracle_c, tile, batch, rows):
+    """Batch boundaries anywhere in a token tile: tiles of 240 tokens start on odd multiples of 16, so their
+    32-token chunks can hold the last rows of one batch and the first of the next."""
+    mode, k, n = 6, 96, 136
+    qweight, scales = oracle.make_weight(n, k, mode, seed=5)
+    op = sdk.PackedLinear.prepare(torch.from_numpy(qweight), torch.from_numpy(scales), None, mode).to(DEV)
+    x = oracle.make_activation(batch * rows, k, seed=rows).reshape(batch, rows, k)
+    g = torch.Generator().manual_seed(batch)
+    gate, residual = torch.randn(batch, n, generator=g).to(torch.bfloat16), torch.randn(batch, rows, n, generator=g).to(torch.bfloat16)
+    got = residual.to(DEV).clone()
+    with option(backend, "token_tile", tile):
+        op.forward_fused(x.to(DEV), None, gate=gate.to(DEV), residual=got)
+    q, sa = oracle.quantize_lift(x.reshape(-1, k), mode)
+    acc = oracle.gemm_int32(q, oracle.slide_weight(qweight, mode), batch * rows)
+    expect = oracle_c.epilogue_gated(acc, sa, scales, None, bits(gate), rows, bits(residual))
+    assert np.array_equal(bits(got).reshape(-1, n), expect)
+    assert backend.device_status() == 0
 
 
 def test_gated_accumulation_argument_errors(sdk, backend, oracle):
