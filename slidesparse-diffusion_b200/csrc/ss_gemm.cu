@@ -52,6 +52,7 @@ struct KernelArgs {
   int debug;                       // diagnostics: bit 0 no MMAs, 1 no epilogue work, 2 no TMA stores, 3 TMEM loads only
   unsigned long long* probe;       // diagnostics: cluster 0 writes {cycles of its tile loop, stages}
   int out_evict_first;             // TMA stores of the output carry the L2 evict_first hint
+  int prefetch_residual;           // gated accumulation: a tile's residual is asked for while its MMAs run
   int32_t* split_sum;              // split schedule: the clusters' slabs for pieces of shared tiles
   int* split_ticket;               // split schedule: arrivals per epilogue warp of a shared tile (zero between launches)
 };
@@ -361,6 +362,12 @@ int launch_pair_t(const GemmArgs& a, DeviceInfo* dev, int tile_index, cudaStream
   // 16384 x 3072 -> 12288 (403 MB out), -1 % on 4096 x 3072 -> 12288 (101 MB), nothing below; a
   // smaller output is left for the kernel that consumes it
   k.out_evict_first = 2 * a.m * a.n >= (63ll << 20) ? 1 : 0;
+  // A gated output far larger than L2 is read, added to and written back in HBM.  Left to the reductions, the
+  // reads begin when a tile is done; asked for at its start they overlap its MMAs.  Pays while the HBM time of
+  // a tile exceeds its MMA time, up to ten blocks of lifted columns: 99 drawn shapes by number of blocks, time with
+  // over time without: 4..8 0.81 .. 0.98, 9 0.91 .. 0.98, 10 0.87 .. 1.00, 11 1.00 .. 1.08, 13 1.04 .. 1.15 (the
+  // lines are pushed out again before they are used).  8640 x 512 -> 15728 (2:4) 142 -> 124 us, 8192 wide 77 -> 64.
+  k.prefetch_residual = k.out_evict_first && a.pk / kBlockK <= 10 ? 1 : 0;
   k.split_sum = nullptr;
   k.split_ticket = nullptr;
   DeviceInfo::SplitArea* split_area = nullptr;

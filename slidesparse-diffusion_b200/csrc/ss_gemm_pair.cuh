@@ -571,6 +571,11 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       if constexpr (ADDEND) {
         if (mine > 0) load_addend(half);
       }
+      if constexpr (GATED) {
+        if (args.prefetch_residual && lane == 0 && ch_w < args.n) {
+          for (int i = 0; i < mine; ++i) ptx::tma_prefetch_2d(&map_out, ch_w, tok0 + (half + kPairSub * i) * 32);
+        }
+      }
       // split schedule: this warp's chunk i of a slab into registers
       auto fetch = [&](uint32_t (&r)[32], const uint4* src, int i) {
 #pragma unroll

@@ -161,6 +161,25 @@ def test_gate_of_every_batch_in_every_tile(sdk, backend, oracle, oracle_c, tile,
     assert backend.device_status() == 0
 
 
+@pytest.mark.parametrize("mode,k,tile", [(4, 512, 0), (6, 844, 240), (4, 1280, 128), (8, 936, 0)])
+def test_gated_accumulation_of_a_large_output(sdk, backend, oracle, oracle_c, mode, k, tile):
+    """Outputs beyond half of the L2, where a tile's residual is prefetched up to ten blocks of lifted columns
+    (here 4, 9, 10 and 11): the same bits, ragged last token and channel tiles, every kernel form."""
+    batch, rows, n = 2, 2272, 7480
+    qweight, scales = oracle.make_weight(n, k, mode, seed=k)
+    op = sdk.PackedLinear.prepare(torch.from_numpy(qweight), torch.from_numpy(scales), None, mode).to(DEV)
+    gen = torch.Generator(device=DEV).manual_seed(k)
+    make = lambda *shape: torch.randn(*shape, generator=gen, device=DEV).to(torch.bfloat16)
+    x, gate, residual = make(batch, rows, k), make(batch, n), make(batch, rows, n)
+    q, sa = backend.quantize_lift_fused(x, mode, backend.Prologue("none"))
+    acc = backend.gemm_int32(q, op.packed, op.metadata, batch * rows, n)
+    expect = oracle_c.epilogue_gated(acc.cpu().numpy(), sa.cpu().numpy(), scales, None, bits(gate), rows, bits(residual))
+    with option(backend, "token_tile", tile):
+        op.forward_fused(x, None, gate=gate, residual=residual)
+    assert np.array_equal(bits(residual).reshape(-1, n), expect.reshape(-1, n))
+    assert backend.device_status() == 0
+
+
 def test_gated_accumulation_argument_errors(sdk, backend, oracle):
     k, n = 128, 64
     qweight, scales = oracle.make_weight(n, k, 4, seed=1)
