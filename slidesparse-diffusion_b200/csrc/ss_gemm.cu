@@ -551,17 +551,27 @@ int check_args(const GemmArgs& a) {
 struct Choice { int nt; int res_stages; bool split; };
 Choice choose(const GemmArgs& a, int sms, bool split_allowed) {
   const Options& opt = options();
+  // the half chunk of the 240-token tile exists in the TMA-store epilogues only
+  const bool whole_chunks_only = a.peer_count > 0;
+  const TilePick whole = pick_pair_token_tile(a.m, a.pn, a.pk, sms, whole_chunks_only);
   if (opt.resident && !a.int32_out && !a.addend && a.peer_count == 0 && opt.token_tile == 0 && tma_store_ok(a)) {
     // prefer the token tile that needs fewer rounds of the clusters that share a channel tile
     const int s224 = resident_stages<224>(a, sms), s192 = resident_stages<192>(a, sms);
     const int64_t tiles_ch2 = (a.pn + 2 * kTileCh - 1) / (2 * kTileCh), group = (sms / 2) / (tiles_ch2 ? tiles_ch2 : 1);
     auto rounds = [&](int nt) { const int64_t t = (a.m + nt - 1) / nt; return (t + group - 1) / group; };
-    if (s224 && (!s192 || rounds(224) * 224 <= rounds(192) * 192)) return {224, s224, false};
-    if (s192) return {192, s192, false};
+    const int nt = s224 && (!s192 || rounds(224) * 224 <= rounds(192) * 192) ? 224 : s192 ? 192 : 0;
+    // Its clusters are a multiple of the channel tiles (40 channel tiles occupy 40 of 74 clusters), so it is
+    // compared by cost, at the streaming form's costs per tile.  237 drawn shapes of 4 to 10 blocks, its time over
+    // the streaming form's, by the ratio of costs, plain / gated: up to 1.1 0.87 .. 1.03 / 0.91 .. 1.05 (6016 x 616 ->
+    // 9288, 4:6: 42.0 against 48.2 us); 1.1 to 1.3 mean 1.02 / 1.03; above mean 1.18 / 1.14 (12928 x 696 -> 10000, 2:4:
+    // 117.9 against 77.1 us).
+    if (nt) {
+      const int i = nt == 224 ? 2 : 1;
+      static_assert(kTiles[1] == 192 && kTiles[2] == 224, "tiles of the resident form");
+      const double cost = static_cast<double>(rounds(nt)) * (static_cast<double>(a.pk / kBlockK) * kPerBlock[i] + kPerTile[i]);
+      if (cost <= 1.1 * whole.cost) return {nt, nt == 224 ? s224 : s192, false};
+    }
   }
-  // the half chunk of the 240-token tile exists in the TMA-store epilogues only
-  const bool whole_chunks_only = a.peer_count > 0;
-  const TilePick whole = pick_pair_token_tile(a.m, a.pn, a.pk, sms, whole_chunks_only);
   // the split schedule: plain aligned BF16 output only, at least two stages per tile, and worth its
   // extra trip through global memory by the cost model (or forced)
   if (split_allowed && opt.split != 0 && a.allow_split && opt.store == 1 && !a.int32_out && !a.addend && !a.gate &&

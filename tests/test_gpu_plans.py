@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import bits, expected_bits, prepare_case, ptr
+from gpu_util import bits, expected_bits, option, prepare_case, ptr
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -142,3 +142,16 @@ def test_configure_reports_the_kernel_resources(sdk, backend, oracle):
     assert lib.ss_gemm_resources(4096, 4608, 1152, out, 8) == 0 and out[5] in (192, 224)    # the weights-resident form
     assert lib.ss_gemm_resources(0, 1, 128, out, 8) == backend.SS_E_ARG
     assert lib.ss_gemm_resources(1, 1, 100, out, 8) == backend.SS_E_ARG
+
+
+@pytest.mark.parametrize("m,n,pk,resident", [(4096, 4608, 1152, True), (6016, 9288, 896, True),
+                                             (12928, 10000, 768, False), (5376, 9632, 896, False)])
+def test_weights_resident_form_where_it_fills_the_clusters(backend, m, n, pk, resident):
+    """40 channel tiles would occupy 40 of 74 clusters: such shapes take the streaming form."""
+    chosen, streaming = (ctypes.c_int64 * 8)(), (ctypes.c_int64 * 8)()
+    torch.zeros(1, device=DEV)
+    lib = backend.library()
+    assert lib.ss_gemm_resources(m, n, pk, chosen, 8) == 0
+    with option(backend, "resident", 0):
+        assert lib.ss_gemm_resources(m, n, pk, streaming, 8) == 0
+    assert (list(chosen) != list(streaming)) == resident
