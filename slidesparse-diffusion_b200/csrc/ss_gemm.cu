@@ -248,6 +248,10 @@ DeviceInfo::SplitArea* split_workspace(DeviceInfo* dev, cudaStream_t stream, boo
 constexpr int kTiles[kTileCount] = {128, 192, 224, 240, 256};
 constexpr double kPerBlock[kTileCount] = {252.0, 331.0, 344.0, 351.0, 382.0};
 constexpr double kPerTile[kTileCount] = {759.0, 1098.0, 1563.0, 1726.0, 2058.0};
+// A gated epilogue takes longer, and the tile of 256 exposes it.  Over 360 drawn gated shapes the choice costs 1.3 %
+// more than the best tile per shape with this constant, 1.5 % without (4096 x 2048 -> 15360, 2:4: tile 256 86.9 us,
+// tile 240, taken now, 76.8).
+constexpr double kGatedPerTile256 = 1000.0;
 
 // Split schedule (see Walk in ss_gemm_pair.cuh): the clusters share the tiles x stages evenly, so a
 // launch costs tiles / clusters (not rounded up) tile costs, plus what the shared tiles cost: every
@@ -259,7 +263,7 @@ constexpr double kPerTile[kTileCount] = {759.0, 1098.0, 1563.0, 1726.0, 2058.0};
 constexpr double kSplitExtra = 11000.0;
 
 struct TilePick { int nt; double cost; };
-TilePick pick_pair_token_tile(int64_t m, int64_t pn, int64_t pk, int sms, bool whole_chunks_only, bool split = false) {
+TilePick pick_pair_token_tile(int64_t m, int64_t pn, int64_t pk, int sms, bool whole_chunks_only, bool split = false, bool gated = false) {
   const int forced = options().token_tile;
   const int64_t tiles_ch2 = (pn + 2 * kTileCh - 1) / (2 * kTileCh);
   const double num_kb = static_cast<double>(pk / kBlockK);
@@ -270,7 +274,7 @@ TilePick pick_pair_token_tile(int64_t m, int64_t pn, int64_t pk, int sms, bool w
     if (whole_chunks_only && nt % 32) continue;
     if (forced && forced != nt) continue;
     const int64_t tiles = tiles_ch2 * ((m + nt - 1) / nt);
-    const double per_tile = num_kb * kPerBlock[i] + kPerTile[i];
+    const double per_tile = num_kb * kPerBlock[i] + kPerTile[i] + (gated && nt == 256 ? kGatedPerTile256 : 0.0);
     double cost;
     if (split) {
       // with fewer tiles than clusters a tile is shared by many and its last piece adds up many
@@ -553,7 +557,7 @@ Choice choose(const GemmArgs& a, int sms, bool split_allowed) {
   const Options& opt = options();
   // the half chunk of the 240-token tile exists in the TMA-store epilogues only
   const bool whole_chunks_only = a.peer_count > 0;
-  const TilePick whole = pick_pair_token_tile(a.m, a.pn, a.pk, sms, whole_chunks_only);
+  const TilePick whole = pick_pair_token_tile(a.m, a.pn, a.pk, sms, whole_chunks_only, false, a.gate != nullptr);
   if (opt.resident && !a.int32_out && !a.addend && a.peer_count == 0 && opt.token_tile == 0 && tma_store_ok(a)) {
     // prefer the token tile that needs fewer rounds of the clusters that share a channel tile
     const int s224 = resident_stages<224>(a, sms), s192 = resident_stages<192>(a, sms);
