@@ -176,7 +176,7 @@ DeviceInfo* device_info() {
 // Token tile of a launch (256 channels x NT tokens per cluster): the candidate with the smallest
 // rounds x cost-per-tile; ties go to the smaller tile.  Cost of one tile in cycles = blocks of 128
 // lifted columns x per-block cost + per-tile cost, both fitted per token tile (relative least
-// squares, with a constant of 8463 cycles per launch that does not matter to the choice) to GEMM times
+// squares, with a constant of 8463 cycles per launch) to GEMM times
 // measured by CUDA-graph replay over 24 shapes (K' 1024 .. 18432, M 64 .. 16384, weights read from HBM).
 // The per-tile part is the epilogue tail and the barrier round trips; 256 has a single accumulator, so
 // its epilogue is exposed.  On 26 other shapes (K' 512 .. 16000, M 128 .. 16384) the choice costs 0.2 % more
@@ -256,11 +256,18 @@ constexpr double kGatedPerTile256 = 1000.0;
 // Split schedule (see Walk in ss_gemm_pair.cuh): the clusters share the tiles x stages evenly, so a
 // launch costs tiles / clusters (not rounded up) tile costs, plus what the shared tiles cost: every
 // cluster stores one accumulator to global memory at the start of its range and fetches one at the
-// end, where nothing hides it, and the clusters no longer walk K in step (measured over 20 shapes:
-// 5-6 us, of which the last piece's fetch and epilogue are about 2 us).  It therefore pays only when
+// end, where nothing hides it, and the clusters no longer walk K in step.  It therefore pays only when
 // a whole-tile launch would idle most clusters through a long last round, e.g. 2048 x 9728 -> 2432
-// (4:6): 100 tiles of 76 stages on 74 clusters, 42.7 -> 38.3 us.
-constexpr double kSplitExtra = 11000.0;
+// (4:6): 100 tiles of 76 stages on 74 clusters, 56.3 -> 52.3 us with its front-end.  Nor does it pay when the
+// quantised activations fill the L2: its clusters are in as many token tiles at once, and each of them comes
+// from HBM again (5908 x 12288 -> 3280, 4:6, 97 MB: 281 us against 172).
+// Constants by least mean time over 210 drawn shapes, whole and split measured at every tile: 0.7 % above
+// the better of all, 0.9 % without the schedule; 0.9 % with 11000 and a margin of 0.93 on the costs without the
+// launch, as fitted beside the costs of the loop with a metadata warp (35 % lost at worst).
+constexpr double kLaunchCost = 8463.0;             // the fitted costs' constant per launch
+constexpr double kSplitExtra = 8000.0;
+constexpr double kSplitMargin = 0.9;
+constexpr int64_t kSplitMaxActivations = 64ll << 20;
 
 struct TilePick { int nt; double cost; };
 TilePick pick_pair_token_tile(int64_t m, int64_t pn, int64_t pk, int sms, bool whole_chunks_only, bool split = false, bool gated = false) {
@@ -581,7 +588,8 @@ Choice choose(const GemmArgs& a, int sms, bool split_allowed) {
   if (split_allowed && opt.split != 0 && a.allow_split && opt.store == 1 && !a.int32_out && !a.addend && !a.gate &&
       a.peer_count == 0 && tma_store_ok(a) && a.pk / kBlockK >= 4) {
     const TilePick shared = pick_pair_token_tile(a.m, a.pn, a.pk, sms, false, true);
-    if (shared.cost > 0 && (opt.split == 1 || shared.cost < 0.93 * whole.cost)) return {shared.nt, 0, true};
+    const bool pays = shared.cost + kLaunchCost < kSplitMargin * (whole.cost + kLaunchCost) && a.m * a.pk <= kSplitMaxActivations;
+    if (shared.cost > 0 && (opt.split == 1 || pays)) return {shared.nt, 0, true};
   }
   return {whole.nt, 0, false};
 }
