@@ -18,6 +18,7 @@ import hashlib
 import json
 import os
 import subprocess
+import warnings
 from pathlib import Path
 
 import torch
@@ -60,7 +61,8 @@ def build_native(output=None, arch=ARCH, force=False):
     Compiles csrc/*.cu into <output>/libslidesparse_b200.so with
     `nvcc -gencode arch=compute_100a,code=sm_100a`, csrc/ss_torch.cpp into the operator binding beside
     it with the host compiler, and writes receipt.json (source / library hashes, torch and CUDA
-    versions, the command).  Returns the receipt.  An up-to-date artefact is kept unless force=True.
+    versions, the command).  Returns the receipt.  An artefact of these sources and this torch is kept
+    unless force=True.
     """
     if torch.cuda.is_initialized():
         raise RuntimeError("build in a fresh CPU-only process")
@@ -73,7 +75,7 @@ def build_native(output=None, arch=ARCH, force=False):
     if not force and target.exists() and binding.exists() and receipt_path.exists():
         old = json.loads(receipt_path.read_text())
         if (old.get("complete") and old.get("source_dependencies") == identity and old.get("library_sha") == sha(target)
-                and old.get("binding_sha") == sha(binding)):
+                and old.get("binding_sha") == sha(binding) and _built_for_this_torch(old)):
             return old
     nvcc = str(Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "bin/nvcc")
     cmd = [nvcc, "-std=c++17", "-O3", "--shared", "-Xcompiler", "-fPIC", "-lineinfo", "-Xptxas=-v",
@@ -89,6 +91,11 @@ def build_native(output=None, arch=ARCH, force=False):
                    compile_log_sha=sha(log), cuda_initialized=torch.cuda.is_initialized())
     receipt_path.write_text(json.dumps(receipt, indent=2) + "\n")
     return receipt
+
+
+def _built_for_this_torch(receipt):
+    """The operator binding holds torch's C++ types: it belongs to the torch (and CUDA) it was compiled against."""
+    return (receipt.get("torch"), receipt.get("cuda")) == (torch.__version__, torch.version.cuda)
 
 
 def _binding_command(directory, target):
@@ -196,13 +203,27 @@ def load_native(directory=None):
         if _loaded_sha != receipt["library_sha"]:
             raise RuntimeError("a different native binary is already loaded in this process")
         return receipt
-    binding = directory / BINDING_LIBRARY_NAME
-    if binding.exists() and receipt.get("binding_sha") != sha(binding):
-        raise ValueError("operator binding differs from its receipt")
+    binding = _usable_binding(directory, receipt)
     _lib = _declare(ctypes.CDLL(str(target)))
     _loaded_sha = receipt["library_sha"]
-    _register_ops(binding if binding.exists() else None)
+    _register_ops(binding)
     return receipt
+
+
+def _usable_binding(directory, receipt):
+    """Path of the operator binding in `directory`, or None (operators through ctypes, which need no torch
+    types) where there is none for this torch."""
+    binding = directory / BINDING_LIBRARY_NAME
+    if not binding.exists():
+        return None
+    if receipt.get("binding_sha") != sha(binding):
+        raise ValueError("operator binding differs from its receipt")
+    if not _built_for_this_torch(receipt):
+        warnings.warn(f"{binding} was built for torch {receipt.get('torch')} with CUDA {receipt.get('cuda')}, this is "
+                      f"{torch.__version__} with {torch.version.cuda}: operators go through ctypes, at 20 to 30 us more "
+                      "host time a call; rebuild with build_native()", RuntimeWarning, stacklevel=3)
+        return None
+    return binding
 
 
 def library():
