@@ -204,9 +204,10 @@ def load_native(directory=None):
             raise RuntimeError("a different native binary is already loaded in this process")
         return receipt
     binding = _usable_binding(directory, receipt)
-    _lib = _declare(ctypes.CDLL(str(target)))
-    _loaded_sha = receipt["library_sha"]
+    lib = _declare(ctypes.CDLL(str(target)))
     _register_ops(binding)
+    # only now: a load that failed on the way can be tried again
+    _lib, _loaded_sha = lib, receipt["library_sha"]
     return receipt
 
 
@@ -750,10 +751,20 @@ def _register_ops(binding):
     global _ops_registered
     if _ops_registered:
         return
-    _ops_registered = True
-    Library = torch.library.Library
+    # the steps that can fail come first and leave nothing behind: another library in this process may define
+    # these names (its operators must not get this binding's kernels), the binding may not load
+    libraries = []
+    try:
+        for name in ("sdacc_dualscale_sm80", "sdacc_mild_projection_sm80", "sdacc_prepared_projection_sm80", "slidesparse_b200"):
+            libraries.append(torch.library.Library(name, "DEF"))
+        if binding is not None:
+            torch.ops.load_library(str(binding))
+    except Exception:
+        for library in libraries:
+            library._destroy()
+        raise
+    dual, mild, prepared, own = libraries
 
-    dual = Library("sdacc_dualscale_sm80", "DEF")
     dual.define("pack_cpu(Tensor weight,int padded_k)->(Tensor,Tensor)")
     dual.define("configure(Tensor anchor,int config,bool has_addend=False)->int[]")
     dual.define("run(Tensor q,Tensor packed,Tensor metadata,Tensor sa,Tensor sw,Tensor bias,int m,int n,"
@@ -761,7 +772,6 @@ def _register_ops(binding):
     dual.impl("pack_cpu", lambda weight, padded_k: pack_weight(weight, padded_k), "CPU")
     dual.impl("configure", _configure, "CUDA")
 
-    mild = Library("sdacc_mild_projection_sm80", "DEF")
     proj = ("(Tensor input,Tensor packed,Tensor metadata,Tensor scales,Tensor bias,int group,int n,int config,"
             "Tensor? output_addend=None)->Tensor")
     mild.define("quantize_packed16(Tensor input,int group)->(Tensor,Tensor)")
@@ -771,7 +781,6 @@ def _register_ops(binding):
     mild.define("projection" + proj)
     mild.define("projection_scalar" + proj)
 
-    prepared = Library("sdacc_prepared_projection_sm80", "DEF")
     prep = ("(Tensor packed,Tensor metadata,Tensor scales,Tensor bias,int k,int m,int n,int group,int config,"
             "bool packed16)->int")
     for name in ("prepare_direct2", "prepare_singlepatch", "prepare"):
@@ -782,7 +791,6 @@ def _register_ops(binding):
     prepared.define("release(int handle)->()")
     prepared.impl("release", _release, "CompositeExplicitAutograd")
     prepared.impl("resources", _resources, "CompositeExplicitAutograd")
-    _libraries.extend([dual, mild, prepared])
 
     @torch.library.register_fake("sdacc_dualscale_sm80::run")
     def _fake_run(q, packed, metadata, sa, sw, bias, m, n, config, output_addend=None):
@@ -800,7 +808,6 @@ def _register_ops(binding):
 
     # additions of this library (no counterpart in the reference): the projection with element-wise
     # neighbours fused in, as operators so that callers using them can still be compiled
-    own = Library("slidesparse_b200", "DEF")
     weights = "Tensor packed,Tensor metadata,Tensor scales,Tensor bias,int group,int n"
     pro = "int prologue,Tensor? shift,Tensor? scale,float eps"
     own.define(f"projection_fused(Tensor input,{pro},{weights},Tensor? output_addend=None)->Tensor")
@@ -820,9 +827,7 @@ def _register_ops(binding):
         _projection_fused_impl(input, _prologue_of(prologue, shift, scale, eps), packed, metadata, scales, bias, group, n,
                                None, gate, residual)
 
-    if binding is not None:
-        torch.ops.load_library(str(binding))
-    else:
+    if binding is None:
         dual.impl("run", _run, "CUDA")
         # One front-end serves all three reference variants: they produce identical bits.
         mild.impl("quantize", _quantize, "CUDA")
@@ -834,7 +839,6 @@ def _register_ops(binding):
         own.impl("gate_add", lambda x, gate, y: torch.addcmul(x, gate[:, None], y), "CompositeImplicitAutograd")
         own.impl("projection_fused", _op_fused, "CUDA")
         own.impl("projection_fused_accumulate_", _op_fused_accumulate, "CUDA")
-    _libraries.append(own)
 
     @torch.library.register_fake("slidesparse_b200::projection_fused")
     def _fake_fused(input, prologue, shift, scale, eps, packed, metadata, scales, bias, group, n, output_addend=None):
@@ -848,3 +852,6 @@ def _register_ops(binding):
     @torch.library.register_fake("slidesparse_b200::projection_fused_accumulate_")
     def _fake_fused_accumulate(residual, input, prologue, shift, scale, eps, packed, metadata, scales, bias, group, n, gate):
         return None
+
+    _libraries.extend(libraries)
+    _ops_registered = True

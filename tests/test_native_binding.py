@@ -75,3 +75,44 @@ with warnings.catch_warnings(record=True) as seen:
 print(json.dumps(dict(native=native(), warned=[str(w.message) for w in seen if "rebuild" in str(w.message)])))
 ''', copy(**changes))
     assert not result["native"] and len(result["warned"]) == 1
+
+
+def test_failed_load_leaves_nothing_behind(backend, copy):
+    """A binding that cannot be loaded, twice, then a good directory in the same process."""
+    broken = copy(name="broken")
+    (broken / backend.BINDING_LIBRARY_NAME).write_bytes(b"not a library")
+    receipt = json.loads((broken / "receipt.json").read_text())
+    receipt["binding_sha"] = backend.sha(broken / backend.BINDING_LIBRARY_NAME)
+    (broken / "receipt.json").write_text(json.dumps(receipt))
+    result = run(r'''
+errors = []
+for _ in range(2):
+    try:
+        package.load_native(sys.argv[2])
+        errors.append("")
+    except OSError as error:
+        errors.append(str(error))
+package.load_native(sys.argv[3])
+print(json.dumps(dict(errors=errors, native=native())))
+''', broken, copy(name="good"))
+    assert all(result["errors"]) and result["native"]
+
+
+def test_names_taken_by_another_library_leave_nothing_behind():
+    """The reference's own extension in the same process defines the same operator names."""
+    result = run(r'''
+other = torch.library.Library("sdacc_prepared_projection_sm80", "DEF")
+errors = []
+for _ in range(2):
+    try:
+        package.load_native()
+        errors.append("")
+    except RuntimeError as error:
+        errors.append(str(error))
+other.define("run(Tensor input,int handle,int n)->Tensor")
+untouched = not torch._C._dispatch_has_kernel_for_dispatch_key("sdacc_prepared_projection_sm80::run", "CUDA")
+other._destroy()
+package.load_native()
+print(json.dumps(dict(errors=errors, native=native(), untouched=untouched)))
+''')
+    assert all(result["errors"]) and result["native"] and result["untouched"]
