@@ -2,11 +2,12 @@
 
 Host-side mirror of `sdacc/w8a8_slidesparse/backend.py` (build_native :17-70, load_native
 :73-118).  The native artefact is a thin C-ABI shared library (include/slidesparse_b200.h) built
-with nvcc for sm_100a only -- no CUTLASS, no Triton, no second backend, no CPU fallback: every
-operator below raises if the library is missing.  Beside it lies a second library built by the host
-compiler from csrc/ss_torch.cpp, which binds the operators of the forward path to that C ABI without
-going through Python (an eager call took 33-40 us of host time through ctypes); a directory that
-holds the C library alone binds the same operators through ctypes.
+with nvcc for sm_100a only -- no CUTLASS, no Triton, no CPU fallback: every operator that runs this
+library's kernels raises if it is missing.  Beside it lies a second library built by the host compiler
+from csrc/ss_torch.cpp, which binds the operators of the forward path to that C ABI without going
+through Python (an eager call took 33-40 us of host time through ctypes).  A directory that holds the C
+library alone, or a binding compiled against another torch, binds the same operators to the same
+kernels through ctypes, with a warning.
 
 The operators keep the reference's names and schemas (csrc/dualscale_sm80.cu:400-406,
 csrc/projection_sm80.cu:154-169, csrc/graph_projection.cuh:178-195) so callers that look them up
@@ -216,6 +217,8 @@ def _usable_binding(directory, receipt):
     types) where there is none for this torch."""
     binding = directory / BINDING_LIBRARY_NAME
     if not binding.exists():
+        warnings.warn(f"{binding} is missing: operators go through ctypes, at 20 to 30 us more host time a call; copy it "
+                      "beside the library, or run build_native()", RuntimeWarning, stacklevel=3)
         return None
     if receipt.get("binding_sha") != sha(binding):
         raise ValueError("operator binding differs from its receipt")

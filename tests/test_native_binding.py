@@ -116,3 +116,18 @@ package.load_native()
 print(json.dumps(dict(errors=errors, native=native(), untouched=untouched)))
 ''')
     assert all(result["errors"]) and result["native"] and result["untouched"]
+
+
+def test_missing_binding_is_said_and_a_whole_copy_is_native(backend, copy):
+    """The C library alone still binds every operator, but not without a word: its calls cost more host time."""
+    body = r'''
+with warnings.catch_warnings(record=True) as seen:
+    warnings.simplefilter("always")
+    package.load_native(sys.argv[2])
+print(json.dumps(dict(native=native(), warned=[str(w.message) for w in seen if backend.BINDING_LIBRARY_NAME in str(w.message)],
+                      defined=hasattr(torch.ops.slidesparse_b200, "projection_fused"))))
+'''
+    alone = run(body, copy((backend.LIBRARY_NAME,), name="alone"))
+    assert not alone["native"] and alone["defined"] and len(alone["warned"]) == 1
+    whole = run(body, copy(name="whole"))
+    assert whole["native"] and whole["defined"] and not whole["warned"]
