@@ -9,11 +9,13 @@
 // ss_micro_mma_rate settles at 127.5 operand bytes per clock whatever N is; A is half as wide after
 // compression, B is not).  No multicast load is involved.  What bounds the pair kernel is measured
 // too, not assumed: first the two single threads that drive the pipeline (TMA issue, MMA
-// issue, commits), now the round trip of the four-stage ring; see the diagnostics entry
-// ss_micro_pair_rate and the counters a -DSS_TIMELINE build keeps.
+// issue, commits), then the round trip of the four-stage ring, now the bytes that the epilogue stores
+// beside the main loop (token tile 224, 448 tensor cycles a stage: 480 without stores, 600 with them); see
+// the diagnostics entry ss_micro_pair_rate and the counters a -DSS_TIMELINE build keeps.
 //
 // Roles per CTA: warp 0 TMA producer, warp 1 MMA and metadata-copy issuer (rank 0 only; also allocates
-// TMEM), warps 2..9 epilogue (two per TMEM lane quadrant); warp 10 has none.
+// TMEM), warps 2..9 epilogue (two per TMEM lane quadrant); warp 10 has none, and stays because the block size is
+// a result of the resource queries.
 //
 // Protocol (rank = %cluster_ctarank):
 //   full[s]      lives in rank 0 only.  Rank 0's producer posts the byte count of BOTH CTAs'
@@ -23,7 +25,7 @@
 //                both producers see the stage free at the same time.
 //   acc_full[b]  one copy per CTA, multicast commit; acc_empty[b] lives in rank 0 and counts the
 //                16 epilogue warps of the pair (rank 1 arrives through shared::cluster).
-// Every wait on these barriers is bounded (ptx::mbar_wait): a wait that runs out records the role
+// Every wait on these barriers is bounded (ptx::mbar_wait, mbar_wait_warp): a wait that runs out records the role
 // in the device status word and the role winds down.
 #pragma once
 
@@ -184,7 +186,7 @@ struct PairResident {
     const int stages = room / T::kBBytes;
     return stages < kStages ? 0 : kStages;
   }
-  static constexpr int kStages = 4;     // activation stages of the resident form (the MMA loop is unrolled over them)
+  static constexpr int kStages = 4;     // activation stages of the resident form
   static int smem_bytes(int slabs) { return slabs * T::kABytes + kStages * T::kBBytes + kFixed; }
 };
 
@@ -352,7 +354,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (rank 0 only)
     // A rolled loop: one copy of the stage's code, short enough to stay in the instruction caches that
-    // eleven warps in four different loops share.
+    // ten warps in three different loops share.
     if (rank == 0) {
       const bool leader = ptx::elect_one();
       constexpr uint32_t idesc = (1u << 2) | (2u << 4) | (1u << 7) | (1u << 10) |
@@ -375,8 +377,8 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       const bool issue_mma = (args.debug & 1) == 0;
       long long probe_begin = 0;
       uint32_t probe_stages = 0, last_buf = 0, last_use = 0, tl = 0;
-      long long pf_acc = 0, pf_ready = 0, pf_mma = 0, pf_commit = 0, pf_peek = 0;
-      (void)pf_acc; (void)pf_ready; (void)pf_mma; (void)pf_commit; (void)pf_peek;
+      long long pf_acc = 0, pf_ready = 0, pf_mma = 0, pf_commit = 0;
+      (void)pf_acc; (void)pf_ready; (void)pf_mma; (void)pf_commit;
       if constexpr (RES) {
         // once per cluster: metadata of the whole K extent from its staging area into TMEM
         if (tile_first < num_tiles) {
@@ -454,7 +456,7 @@ sparse_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         last_use = acc_it / T::kAccBufs;
       }
       SS_PF_STORE(8, pf_acc); SS_PF_STORE(9, pf_ready); SS_PF_STORE(10, pf_mma); SS_PF_STORE(11, pf_commit);
-      SS_PF_STORE(12, pf_peek); SS_PF_STORE(13, static_cast<long long>(probe_stages));
+      SS_PF_STORE(13, static_cast<long long>(probe_stages));
       if (probe && ok && probe_stages > 0) {
         // the last tile's accumulator is complete when its barrier (this CTA's copy) flips
         if (!ptx::mbar_wait_warp(&bar_acc_full[last_buf], last_use & 1u, args.wait_ns)) ok = false;
